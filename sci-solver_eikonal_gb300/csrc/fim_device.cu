@@ -54,7 +54,14 @@ namespace {
 // ---------------------------------------------------------------------------
 // device control block
 // ---------------------------------------------------------------------------
+// Barrier of a resident loop kernel's CTAs: arrivals so far, and whether a bounded wait
+// gave up.
+struct GridBar {
+  unsigned count, fail;
+};
+
 struct Ctl {
+  GridBar bar;
   int iter;       // completed outer iterations
   int max_iters;
   int nact;       // active blocks this iteration
@@ -126,6 +133,7 @@ struct DevArgs {
   const int* slot_f64;
   const double* coef64;
   int* inst_fail;
+  int* inst_unreached;  // 2D loop kernel: vertices of the instance still at LARGENUM
   int ninst;
   const int* inst_vbeg;  // renumbered vertex range of every instance (ninst + 1)
   const int2* chunks;    // (instance, first vertex) of every 2D vertex-test chunk
@@ -1703,6 +1711,8 @@ size_t smem_bytes_slot2d(int max_slots_pad, int max_local, int max_owned) {
   return (n + 15) & ~(size_t)15;
 }
 
+#include "loop2d.cuh"
+
 // ===========================================================================
 // 3D: commit visit outputs (CopyOutBack), mark visited blocks, queue the
 // neighbours of converged blocks for a check and carry unconverged blocks over.
@@ -2441,6 +2451,11 @@ struct DeviceSolve::Impl {
   int* inst_nnext = nullptr;
   int* inst_fail = nullptr;
   int* inst_maxit = nullptr;
+  int* inst_unreached = nullptr;
+  unsigned char* stage = nullptr;  // loop kernels: control block and the solve's inputs
+  size_t stage_cap = 0;
+  std::vector<unsigned char> h_stage;
+  Ctl* last_ctl = nullptr;  // the control block of the last solve
   int* cand = nullptr;        // 2 x nb check candidates (checks inside the sweep kernel)
   int* inst_swept = nullptr;  // per instance: blocks swept this iteration
   int* inst_ncand = nullptr;  // per instance: check candidates queued this iteration
@@ -2506,6 +2521,10 @@ struct DeviceSolve::Impl {
   }
   size_t smem = 0;
   int grid_visit = 0, grid_aux = 0;
+  const void* loop_func = nullptr;  // 2D loop kernel of the layout and its launch shape, chosen at its first solve
+  int loop_grid = 0, loop_threads = 0;
+  size_t loop_smem = 0;
+  void* opt_stream = nullptr;  // the solver's stream
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   int max_slots_pad = 0, max_local = 0, max_owned = 0;
   struct Launch {
@@ -2520,7 +2539,7 @@ struct DeviceSolve::Impl {
     void* ps[] = {blocks, coef, lv, halo, nbr_off, nbr, vblock, perm, Ta, Tb, Tinit, prev, conv,
                   stampA, stampC, visited, list0, list1, list_new, ctl, hist, ktime, out_tmp,
                   blk_inst, inst_done, inst_iters, inst_nnext, inst_fail, inst_maxit, seed_ids,
-                  cand, inst_swept, inst_ncand, slot_f64, coef64, res_cand, inst_vbeg, chunks, chk_memo, hsb, hs64, hsu64};
+                  cand, inst_swept, inst_ncand, inst_unreached, stage, slot_f64, coef64, res_cand, inst_vbeg, chunks, chk_memo, hsb, hs64, hsu64};
     for (void* p : ps)
       if (p) cudaFree(p);
     hsb = nullptr;
@@ -2543,12 +2562,19 @@ struct DeviceSolve::Impl {
     list1 = nullptr; list_new = nullptr; ctl = nullptr; hist = nullptr; ktime = nullptr; out_tmp = nullptr;
     blk_inst = nullptr; inst_done = nullptr; inst_iters = nullptr; inst_nnext = nullptr; inst_fail = nullptr;
     inst_maxit = nullptr;
+    inst_unreached = nullptr;
+    stage = nullptr;
+    stage_cap = 0;
     cand = nullptr; inst_swept = nullptr; inst_ncand = nullptr;
     hist_cap = 0;
     ktime_cap = 0;
+    loop_func = nullptr;
     drop_graph();
   }
+  void fill_args(DevArgs& a, const Layout& L, int sweeps, int hcap, bool serve, bool tele) const;
   std::string build_graph(const Layout& L, int sweeps, int threads, int hcap, bool serve);
+  std::string choose_loop2d(const Layout& L);
+  std::string run_loop2d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap);
   void drop_graph() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -2559,40 +2585,136 @@ struct DeviceSolve::Impl {
   }
 };
 
+// The kernels' view of the uploaded layout and the solver state.
+void DeviceSolve::Impl::fill_args(DevArgs& a, const Layout& L, int sweeps, int hcap, bool serve, bool tele) const {
+  const Impl& P = *this;
+  a = DevArgs{};
+  a.blocks = P.blocks; a.coef = P.coef; a.lv = P.lv; a.halo = P.halo; a.nbr_off = P.nbr_off; a.nbr = P.nbr;
+  a.vblock = P.vblock; a.nb = L.nb; a.nv = L.nv; a.Ta = P.Ta; a.Tb = P.Tb; a.Tinit = P.Tinit; a.prev = P.prev;
+  a.conv = P.conv; a.stampA = P.stampA; a.stampC = P.stampC; a.visited = P.visited; a.list0 = P.list0;
+  a.list1 = P.list1; a.list_new = P.list_new; a.ctl = P.ctl; a.hist = P.hist; a.hist_cap = hcap;
+  a.ktime = tele ? P.ktime : nullptr;
+  a.ktime_cap = tele ? P.ktime_cap : 0;
+  a.fim_sweeps = sweeps; a.max_slots_pad = P.max_slots_pad; a.max_local = P.max_local;
+  a.max_owned = P.max_owned;
+  a.use_cond = 1;
+  a.blk_inst = P.blk_inst; a.inst_done = P.inst_done; a.inst_iters = P.inst_iters;
+  a.inst_nnext = P.inst_nnext; a.inst_fail = P.inst_fail; a.ninst = P.ninst; a.inst_maxit = P.inst_maxit;
+  a.inst_vbeg = P.inst_vbeg;
+  a.chunks = P.chunks;
+  a.nchunks = P.nchunks;
+  a.serve = serve ? 1 : 0;
+  a.pending = P.pending_dev;
+  a.slot_f64 = P.slot_f64;
+  a.coef64 = P.coef64;
+  // (serving clears an instance's memos when admission rewrites its coefficients)
+  a.chk_memo = (L.dim == 3) ? P.chk_memo : nullptr;
+  a.hsb = (L.dim == 3) ? P.hsb : nullptr;
+  a.hs64 = P.hs64;
+  a.hsu64 = P.hsu64;
+  a.cand = P.cand;
+  a.inst_swept = P.inst_swept;
+  a.inst_ncand = P.inst_ncand;
+  a.inst_unreached = P.inst_unreached;
+  if (serve) { a.ktime = nullptr; a.ktime_cap = 0; }
+}
+
+// The loop kernel of a 2D layout and its launch shape.
+//   * One resident CTA per block (k_blocks2d, three lanes per slot) where the GPU holds
+//     them, with as many registers as still let all blocks fit (64, 48, 40 or 32 a
+//     thread), up to five CTAs an SM: 640 blocks took 12.3 us an iteration against
+//     16.0 with lists, 1,849 blocks 3.4 times the lists' time (every CTA meets at every
+//     barrier, most of them with nothing to do).
+//   * Else the active list (k_loop2d).  One solve: a few hundred active blocks, latency
+//     counts, three lanes per slot.  A batch: thousands of active blocks, throughput
+//     counts, one lane per slot (256 icospheres at 32 vertices per block 9.8 ms against
+//     12.5 with three lanes, which load every slot three times).
+// Three lanes need blocks of at most 320 slots (1024 threads).
+std::string DeviceSolve::Impl::choose_loop2d(const Layout& L) {
+  Impl& P = *this;
+  static const void* const resident[] = {(const void*)k_blocks2d<64>, (const void*)k_blocks2d<48>,
+                                         (const void*)k_blocks2d<40>, (const void*)k_blocks2d<32>};
+  const int threads[2] = {(L.max_slots + 9) / 10 * 32, (L.max_slots + 31) & ~31};
+  int dev = 0, nsm = 0, occ = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  P.loop_smem = smem_bytes_loop2d(P.max_local, P.max_owned, true);
+  if (threads[0] <= 1024 && L.nb <= 5 * nsm)
+    for (const void* f : resident) {
+      CK(raise_smem_limit(f, P.loop_smem));
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads[0], P.loop_smem));
+      if ((long long)occ * nsm < L.nb) continue;
+      P.loop_func = f;
+      P.loop_threads = threads[0];
+      P.loop_grid = L.nb;
+      return "";
+    }
+  const bool three = L.ninst <= 1 && threads[0] <= 1024;
+  const void* f = three ? (const void*)k_loop2d<3, 64> : (const void*)k_loop2d<1, 64>;
+  P.loop_threads = threads[three ? 0 : 1];
+  P.loop_smem = smem_bytes_loop2d(P.max_local, P.max_owned, false);
+  CK(raise_smem_limit(f, P.loop_smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, P.loop_threads, P.loop_smem));
+  if (occ < 1) return "loop kernel cannot be resident (shared memory / registers)";
+  P.loop_func = f;
+  P.loop_grid = std::max(1, std::min(occ * nsm, L.nb));
+  return "";
+}
+
+// One 2D solve or batch in k_loop2d, enqueued on the solver's stream: one copy of the
+// inputs, one launch.
+std::string DeviceSolve::Impl::run_loop2d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap,
+                                          int max_iters, int hcap) {
+  Impl& P = *this;
+  cudaStream_t st = (cudaStream_t)opt_stream;
+  DevArgs a;
+  P.fill_args(a, L, 7, hcap, false, opt.telemetry);
+  a.use_cond = 0;
+  const size_t nseed = P.h_seed_ids.size(), nact = P.h_act.size(), ni = (size_t)P.ninst;
+  const size_t o_flags = (sizeof(Ctl) + 127) & ~(size_t)127, o_sync = o_flags + sizeof(GridFlag) * kGridFlags;
+  const size_t o_words = o_sync + sizeof(InstSync) * ni;
+  const size_t bytes = o_words + sizeof(int) * (3 * ni + 1 + nseed + nact);
+  if (bytes > P.stage_cap) {
+    std::string e = dev_alloc(P.stage, bytes + 1024);
+    if (!e.empty()) return e;
+    P.stage_cap = bytes + 1024;
+  }
+  P.h_stage.assign(bytes, 0);
+  Ctl c{};
+  c.max_iters = max_iters;
+  c.nact = (int)nact;
+  std::memcpy(P.h_stage.data(), &c, sizeof(Ctl));
+  int* w = reinterpret_cast<int*>(P.h_stage.data() + o_words);
+  for (size_t i = 0; i < ni; ++i) w[i] = (cap[i] <= 0) ? 1 : P.h_done[i];
+  std::copy(cap.begin(), cap.end(), w + ni);
+  if (L.ninst > 1) std::copy(L.inst_bbeg.begin(), L.inst_bbeg.end(), w + 2 * ni);
+  else w[2 * ni + 1] = L.nb;
+  std::copy(P.h_seed_ids.begin(), P.h_seed_ids.end(), w + 3 * ni + 1);
+  std::copy(P.h_act.begin(), P.h_act.end(), w + 3 * ni + 1 + nseed);
+  CK(cudaMemcpyAsync(P.stage, P.h_stage.data(), bytes, cudaMemcpyHostToDevice, st));
+  a.ctl = P.last_ctl = reinterpret_cast<Ctl*>(P.stage);
+  const int* dw = reinterpret_cast<const int*>(P.stage + o_words);
+  Start2 s2{dw, dw + ni, dw + 3 * ni + 1, dw + 3 * ni + 1 + nseed, (int)nseed, (int)nact, dw + 2 * ni,
+            reinterpret_cast<InstSync*>(P.stage + o_sync), reinterpret_cast<GridFlag*>(P.stage + o_flags), P.h_prev.empty() ? 0 : 1, a.ktime ? 1 : 0};
+  if (!P.h_prev.empty())
+    CK(cudaMemcpyAsync(P.prev, P.h_prev.data(), sizeof(float) * L.nv, cudaMemcpyHostToDevice, st));
+  if (!P.loop_func) {
+    std::string e = P.choose_loop2d(L);
+    if (!e.empty()) return e;
+  }
+  CK(cudaEventRecord(P.ev0, st));
+  void* args[] = {&a, &s2};
+  CK(cudaLaunchCooperativeKernel(P.loop_func, dim3(P.loop_grid), dim3(P.loop_threads), args, P.loop_smem, st));
+  return "";
+}
+
 std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int threads, int hcap, bool serve) {
   Impl& P = *this;
   const bool want_hist = hcap > 0;
   {
     P.drop_graph();
     DevArgs& a = P.args;
-    a = DevArgs{};
-    a.blocks = P.blocks; a.coef = P.coef; a.lv = P.lv; a.halo = P.halo; a.nbr_off = P.nbr_off; a.nbr = P.nbr;
-    a.vblock = P.vblock; a.nb = L.nb; a.nv = L.nv; a.Ta = P.Ta; a.Tb = P.Tb; a.Tinit = P.Tinit; a.prev = P.prev;
-    a.conv = P.conv; a.stampA = P.stampA; a.stampC = P.stampC; a.visited = P.visited; a.list0 = P.list0;
-    a.list1 = P.list1; a.list_new = P.list_new; a.ctl = P.ctl; a.hist = P.hist; a.hist_cap = hcap;
-    a.ktime = P.want_tele ? P.ktime : nullptr;
-    a.ktime_cap = P.want_tele ? P.ktime_cap : 0;
-    a.fim_sweeps = sweeps; a.max_slots_pad = P.max_slots_pad; a.max_local = P.max_local;
-    a.max_owned = P.max_owned;
-    a.use_cond = 1;
-    a.blk_inst = P.blk_inst; a.inst_done = P.inst_done; a.inst_iters = P.inst_iters;
-    a.inst_nnext = P.inst_nnext; a.inst_fail = P.inst_fail; a.ninst = P.ninst; a.inst_maxit = P.inst_maxit;
-    a.inst_vbeg = P.inst_vbeg;
-    a.chunks = P.chunks;
-    a.nchunks = P.nchunks;
-    a.serve = serve ? 1 : 0;
-    a.pending = P.pending_dev;
-    a.slot_f64 = P.slot_f64;
-    a.coef64 = P.coef64;
-    // (serving clears an instance's memos when admission rewrites its coefficients)
-    a.chk_memo = (L.dim == 3) ? P.chk_memo : nullptr;
-    a.hsb = (L.dim == 3) ? P.hsb : nullptr;
-    a.hs64 = P.hs64;
-    a.hsu64 = P.hsu64;
-    a.cand = P.cand;
-    a.inst_swept = P.inst_swept;
-    a.inst_ncand = P.inst_ncand;
-    if (serve) { a.ktime = nullptr; a.ktime_cap = 0; }
+    fill_args(a, L, sweeps, hcap, serve, P.want_tele);
     CK(cudaGraphCreate(&P.graph, 0));
     CK(cudaGraphConditionalHandleCreate(&a.cond, P.graph, 0, 0));
     int dev = 0, nsm = 0;
@@ -2800,6 +2922,7 @@ DeviceSolve::DeviceSolve() : p_(new Impl) {
   cudaGetDevice(&p_->device);
   cudaStream_t s;
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess) stream_ = s;
+  p_->opt_stream = stream_;
   cudaEventCreate(&p_->ev0);
   cudaEventCreate(&p_->ev1);
 }
@@ -3023,7 +3146,7 @@ std::string DeviceSolve::finish_upload(const Layout& L, bool layout_on_device) {
   P.ninst = std::max(L.ninst, 1);
   if (!(e = dev_alloc(P.blk_inst, (size_t)L.nb)).empty()) return e;
   for (int** t : {&P.inst_done, &P.inst_iters, &P.inst_nnext, &P.inst_fail, &P.inst_maxit, &P.inst_swept,
-                  &P.inst_ncand})
+                  &P.inst_ncand, &P.inst_unreached})
     if (!(e = dev_alloc(*t, (size_t)P.ninst)).empty()) return e;
   if (!(e = dev_alloc(P.cand, 2 * (size_t)L.nb)).empty()) return e;
   if (!(e = dev_alloc(P.inst_vbeg, (size_t)P.ninst + 1)).empty()) return e;
@@ -3177,6 +3300,8 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
       }
     }
   }
+  // 2D solves of the reference's seven sweeps run in one resident kernel (k_loop2d)
+  const bool loop2d = L.dim == 2 && sweeps == 7 && !opt.direct_launch && P.max_slots_pad <= 1024;
   // per-instance iteration caps (one cap for all when not given)
   std::vector<int> cap(P.ninst, opt.max_iterations);
   if ((int)opt.inst_max_iterations.size() == P.ninst) cap = opt.inst_max_iterations;
@@ -3199,135 +3324,145 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   }
   if (opt.telemetry || tune_slot >= 0)
     CK(cudaMemsetAsync(P.ktime, 0, sizeof(unsigned long long) * kKStride * (size_t)P.ktime_cap, st));
-  // initial state
-  // initial state built on the device: only the seed ids, the starting blocks and
-  // (when given) the caller's initial values cross from the host
-  if (P.h_seed_ids.size() > P.seed_cap) {
-    if (P.seed_ids) cudaFree(P.seed_ids);
-    P.seed_ids = nullptr;
-    P.seed_cap = std::max<size_t>(P.h_seed_ids.size(), 64);
-    CK(cudaMalloc((void**)&P.seed_ids, sizeof(int) * P.seed_cap));
-  }
-  const float large = (L.dim == 3) ? kLarge3D : kLarge2D;
-  const bool user_prev = !P.h_prev.empty();
-  const int nseed = (int)P.h_seed_ids.size();
-  if (nseed > 0)
-    CK(cudaMemcpyAsync(P.seed_ids, P.h_seed_ids.data(), sizeof(int) * nseed, cudaMemcpyHostToDevice, st));
-  k_init_state<<<std::max(1, std::min(4096, (L.nv + 255) / 256)), 256, 0, st>>>(
-      P.Ta, P.Tb, P.Tinit, user_prev ? nullptr : P.prev, L.nv, large);
-  if (user_prev) CK(cudaMemcpyAsync(P.prev, P.h_prev.data(), sizeof(float) * L.nv, cudaMemcpyHostToDevice, st));
-  CK(cudaMemsetAsync(P.stampA, 0, sizeof(int) * L.nb, st));
-  if (!P.h_act.empty())
-    CK(cudaMemcpyAsync(P.list0, P.h_act.data(), sizeof(int) * P.h_act.size(), cudaMemcpyHostToDevice, st));
-  {
-    const int nact = (int)P.h_act.size();
-    const int n = std::max(nseed, nact);
-    if (n > 0)
-      k_seed_state<<<std::max(1, std::min(1024, (n + 255) / 256)), 256, 0, st>>>(
-          P.seed_ids, nseed, P.Ta, P.Tb, P.Tinit, user_prev ? nullptr : P.prev, P.list0, nact,
-          (L.dim == 2) ? P.stampA : nullptr);
-    CK(cudaGetLastError());
-  }
-  CK(cudaMemsetAsync(P.stampC, 0, sizeof(int) * L.nb, st));
-  CK(cudaMemsetAsync(P.visited, 0, L.nb, st));
-  CK(cudaMemsetAsync(P.conv, 0, sizeof(int) * L.nb, st));
-  // 3D check memos (16 B per slot) hold only for this solve's coefficients and kernel
-  if (L.dim == 3) {
-    if (!P.chk_memo) {
-      std::string e = dev_alloc(P.chk_memo, 2 * (P.coef_n / 6));
-      if (!e.empty()) return e;
-      P.drop_graph();
-    }
-    CK(cudaMemsetAsync(P.chk_memo, 0xff, sizeof(uint4) * 2 * (P.coef_n / 6), st));
-  }
-  {
-    std::vector<int> done(P.h_done);
-    for (int i = 0; i < P.ninst; ++i)
-      if (cap[i] <= 0) done[i] = 1;
-    P.h_maxit = cap;
-    CK(cudaMemcpyAsync(P.inst_done, done.data(), sizeof(int) * P.ninst, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(P.inst_maxit, P.h_maxit.data(), sizeof(int) * P.ninst, cudaMemcpyHostToDevice, st));
-    for (int* t : {P.inst_iters, P.inst_nnext, P.inst_fail, P.inst_swept, P.inst_ncand})
-      CK(cudaMemsetAsync(t, 0, sizeof(int) * P.ninst, st));
-  }
-  stats_.h2d_bytes = (long long)sizeof(float) * P.h_prev.size() + (long long)sizeof(int) * nseed +
+  stats_.h2d_bytes = (long long)sizeof(float) * P.h_prev.size() + (long long)sizeof(int) * P.h_seed_ids.size() +
                      (long long)sizeof(int) * P.h_act.size() + 2ll * sizeof(int) * P.ninst + (long long)sizeof(Ctl);
-  Ctl c{};
-  c.max_iters = max_iters;
-  c.nact = (int)P.h_act.size();
-  CK(cudaMemcpyAsync(P.ctl, &c, sizeof(Ctl), cudaMemcpyHostToDevice, st));
-
-  // (re)build the graph when the launch shape changes; the CTA-size tuning of the
-  // slot kernels measures with the telemetry whatever the option says
-  const bool want_hist = hcap > 0;
-  P.want_tele = opt.telemetry || tune_slot >= 0;
-  if (!P.exec || P.g_sweeps != sweeps || P.g_threads != threads || P.g_hist != want_hist || P.g_histcap != hcap ||
-      P.g_serve != 0 || P.g_tele != P.want_tele) {
-    std::string e = P.build_graph(L, sweeps, threads, hcap, false);
-    if (!e.empty()) return e;
-  }
-  // the device loop from the control block's current state
-  auto run_loop = [&]() -> std::string {
-    if (!opt.direct_launch) {
-      CK(cudaGraphLaunch(P.exec, st));
-      return "";
-    }
-    // the graph's kernels launched one by one, the host reading the control block
-    // between iterations (profilers cannot see kernels inside conditional graphs)
-    DevArgs d = P.args;
-    d.use_cond = 0;
-    for (bool first = true;; first = false) {
-      Ctl h{};
-      CK(cudaMemcpyAsync(&h, P.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-      // the graph's start node's test, then its closes' decision
-      if (h.error || (first ? !has_work(h, d.fused) : h.stop != 0)) break;
-      for (const Impl::Launch& l : P.body) {
-        void* args[2] = {&d, (void*)&l.extra};
-        CK(cudaLaunchKernel(l.func, dim3(l.grid), dim3(l.block), args, l.smem, st));
-      }
-      CK(cudaGetLastError());
-    }
-    return "";
-  };
-  CK(cudaEventRecord(P.ev0, st));
-  {
-    std::string e = run_loop();
-    if (!e.empty()) return e;
-  }
-  // Precision mode acts on its FP64 residual: the blocks owning a vertex that the
-  // FP64 update of its tets would lower run the loop again, every slot in FP64,
-  // until no such vertex is left (or kPolishRounds rounds).  With no tet flagged
-  // the caller asked for FP32 throughout, and nothing is re-visited.
   stats_.polish_rounds = 0;
   stats_.polish_blocks = 0;
-  if (P.prec && P.res_cand && L.flagged_tets > 0) {
-    int dev = 0, nsm = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    for (int round = 0; round < kPolishRounds; ++round) {
-      CK(cudaMemsetAsync(P.res_cand, 0x7f, sizeof(unsigned long long) * L.nv, st));
-      k_residual3d<<<std::max(1, std::min(L.nb, 8 * nsm)), 256, 0, st>>>(P.args, P.res_cand, 1);
-      k_polish_begin<<<1, 256, 0, st>>>(P.args, kPolishIterations);
-      k_polish_mark<<<std::max(1, std::min(4 * nsm, (L.nv + 255) / 256)), 256, 0, st>>>(P.args, P.res_cand, P.stampC,
-                                                                                      -(round + 1), kPolishTol);
+  bool tele = false;  // whether this solve recorded its launches
+  if (loop2d) {
+    std::string e = P.run_loop2d(L, opt, cap, max_iters, hcap);
+    if (!e.empty()) return e;
+    tele = opt.telemetry;
+  } else {
+    P.last_ctl = P.ctl;
+    // initial state
+    // initial state built on the device: only the seed ids, the starting blocks and
+    // (when given) the caller's initial values cross from the host
+    if (P.h_seed_ids.size() > P.seed_cap) {
+      if (P.seed_ids) cudaFree(P.seed_ids);
+      P.seed_ids = nullptr;
+      P.seed_cap = std::max<size_t>(P.h_seed_ids.size(), 64);
+      CK(cudaMalloc((void**)&P.seed_ids, sizeof(int) * P.seed_cap));
+    }
+    const float large = (L.dim == 3) ? kLarge3D : kLarge2D;
+    const bool user_prev = !P.h_prev.empty();
+    const int nseed = (int)P.h_seed_ids.size();
+    if (nseed > 0)
+      CK(cudaMemcpyAsync(P.seed_ids, P.h_seed_ids.data(), sizeof(int) * nseed, cudaMemcpyHostToDevice, st));
+    k_init_state<<<std::max(1, std::min(4096, (L.nv + 255) / 256)), 256, 0, st>>>(
+        P.Ta, P.Tb, P.Tinit, user_prev ? nullptr : P.prev, L.nv, large);
+    if (user_prev) CK(cudaMemcpyAsync(P.prev, P.h_prev.data(), sizeof(float) * L.nv, cudaMemcpyHostToDevice, st));
+    CK(cudaMemsetAsync(P.stampA, 0, sizeof(int) * L.nb, st));
+    if (!P.h_act.empty())
+      CK(cudaMemcpyAsync(P.list0, P.h_act.data(), sizeof(int) * P.h_act.size(), cudaMemcpyHostToDevice, st));
+    {
+      const int nact = (int)P.h_act.size();
+      const int n = std::max(nseed, nact);
+      if (n > 0)
+        k_seed_state<<<std::max(1, std::min(1024, (n + 255) / 256)), 256, 0, st>>>(
+            P.seed_ids, nseed, P.Ta, P.Tb, P.Tinit, user_prev ? nullptr : P.prev, P.list0, nact,
+            (L.dim == 2) ? P.stampA : nullptr);
       CK(cudaGetLastError());
-      Ctl h{};
-      CK(cudaMemcpyAsync(&h, P.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-      if (h.error || h.nact == 0) break;
-      if (P.chk_memo) CK(cudaMemsetAsync(P.chk_memo, 0xff, sizeof(uint4) * 2 * (P.coef_n / 6), st));
+    }
+    CK(cudaMemsetAsync(P.stampC, 0, sizeof(int) * L.nb, st));
+    CK(cudaMemsetAsync(P.visited, 0, L.nb, st));
+    CK(cudaMemsetAsync(P.conv, 0, sizeof(int) * L.nb, st));
+    // 3D check memos (16 B per slot) hold only for this solve's coefficients and kernel
+    if (L.dim == 3) {
+      if (!P.chk_memo) {
+        std::string e = dev_alloc(P.chk_memo, 2 * (P.coef_n / 6));
+        if (!e.empty()) return e;
+        P.drop_graph();
+      }
+      CK(cudaMemsetAsync(P.chk_memo, 0xff, sizeof(uint4) * 2 * (P.coef_n / 6), st));
+    }
+    {
+      std::vector<int> done(P.h_done);
+      for (int i = 0; i < P.ninst; ++i)
+        if (cap[i] <= 0) done[i] = 1;
+      P.h_maxit = cap;
+      CK(cudaMemcpyAsync(P.inst_done, done.data(), sizeof(int) * P.ninst, cudaMemcpyHostToDevice, st));
+      CK(cudaMemcpyAsync(P.inst_maxit, P.h_maxit.data(), sizeof(int) * P.ninst, cudaMemcpyHostToDevice, st));
+      for (int* t : {P.inst_iters, P.inst_nnext, P.inst_fail, P.inst_swept, P.inst_ncand})
+        CK(cudaMemsetAsync(t, 0, sizeof(int) * P.ninst, st));
+    }
+    Ctl c{};
+    c.max_iters = max_iters;
+    c.nact = (int)P.h_act.size();
+    CK(cudaMemcpyAsync(P.ctl, &c, sizeof(Ctl), cudaMemcpyHostToDevice, st));
+
+    // (re)build the graph when the launch shape changes; the CTA-size tuning of the
+    // slot kernels measures with the telemetry whatever the option says
+    const bool want_hist = hcap > 0;
+    P.want_tele = opt.telemetry || tune_slot >= 0;
+    if (!P.exec || P.g_sweeps != sweeps || P.g_threads != threads || P.g_hist != want_hist || P.g_histcap != hcap ||
+        P.g_serve != 0 || P.g_tele != P.want_tele) {
+      std::string e = P.build_graph(L, sweeps, threads, hcap, false);
+      if (!e.empty()) return e;
+    }
+    tele = P.g_tele;
+    // the device loop from the control block's current state
+    auto run_loop = [&]() -> std::string {
+      if (!opt.direct_launch) {
+        CK(cudaGraphLaunch(P.exec, st));
+        return "";
+      }
+      // the graph's kernels launched one by one, the host reading the control block
+      // between iterations (profilers cannot see kernels inside conditional graphs)
+      DevArgs d = P.args;
+      d.use_cond = 0;
+      for (bool first = true;; first = false) {
+        Ctl h{};
+        CK(cudaMemcpyAsync(&h, P.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        // the graph's start node's test, then its closes' decision
+        if (h.error || (first ? !has_work(h, d.fused) : h.stop != 0)) break;
+        for (const Impl::Launch& l : P.body) {
+          void* args[2] = {&d, (void*)&l.extra};
+          CK(cudaLaunchKernel(l.func, dim3(l.grid), dim3(l.block), args, l.smem, st));
+        }
+        CK(cudaGetLastError());
+      }
+      return "";
+    };
+    CK(cudaEventRecord(P.ev0, st));
+    {
       std::string e = run_loop();
       if (!e.empty()) return e;
-      stats_.polish_rounds = round + 1;
-      stats_.polish_blocks += h.nact;
+    }
+    // Precision mode acts on its FP64 residual: the blocks owning a vertex that the
+    // FP64 update of its tets would lower run the loop again, every slot in FP64,
+    // until no such vertex is left (or kPolishRounds rounds).  With no tet flagged
+    // the caller asked for FP32 throughout, and nothing is re-visited.
+    if (P.prec && P.res_cand && L.flagged_tets > 0) {
+      int dev = 0, nsm = 0;
+      CK(cudaGetDevice(&dev));
+      CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+      for (int round = 0; round < kPolishRounds; ++round) {
+        CK(cudaMemsetAsync(P.res_cand, 0x7f, sizeof(unsigned long long) * L.nv, st));
+        k_residual3d<<<std::max(1, std::min(L.nb, 8 * nsm)), 256, 0, st>>>(P.args, P.res_cand, 1);
+        k_polish_begin<<<1, 256, 0, st>>>(P.args, kPolishIterations);
+        k_polish_mark<<<std::max(1, std::min(4 * nsm, (L.nv + 255) / 256)), 256, 0, st>>>(P.args, P.res_cand, P.stampC,
+                                                                                        -(round + 1), kPolishTol);
+        CK(cudaGetLastError());
+        Ctl h{};
+        CK(cudaMemcpyAsync(&h, P.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        if (h.error || h.nact == 0) break;
+        if (P.chk_memo) CK(cudaMemsetAsync(P.chk_memo, 0xff, sizeof(uint4) * 2 * (P.coef_n / 6), st));
+        std::string e = run_loop();
+        if (!e.empty()) return e;
+        stats_.polish_rounds = round + 1;
+        stats_.polish_blocks += h.nact;
+      }
     }
   }
   CK(cudaEventRecord(P.ev1, st));
   CK(cudaStreamSynchronize(st));
   CK(cudaGetLastError());
   Ctl out{};
-  CK(cudaMemcpy(&out, P.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(&out, P.last_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
+  if (out.bar.fail) out.error |= kErrWait;
   cudaEventElapsedTime(&stats_.solve_ms, P.ev0, P.ev1);
   // a trailing iteration that swept nothing (its checks activated no block) is not
   // one of the reference's iterations
@@ -3349,8 +3484,8 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   stats_.fim_kernel_ms = stats_.check_kernel_ms = 0.0f;
   stats_.fim_launches = stats_.check_launches = 0;
   stats_.iter_stats.clear();
-  if (P.g_tele) {
-    std::vector<unsigned long long> kt(kKStride * (size_t)P.ktime_cap);
+  if (tele) {
+    std::vector<unsigned long long> kt(kKStride * (size_t)std::max(1, std::min(out.iter, P.ktime_cap)));
     CK(cudaMemcpy(kt.data(), P.ktime, sizeof(unsigned long long) * kt.size(), cudaMemcpyDeviceToHost));
     double fim = 0, chk = 0;
     int nf = 0, nc = 0;
