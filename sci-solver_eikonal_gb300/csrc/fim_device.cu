@@ -703,13 +703,13 @@ __global__ void __launch_bounds__(1024) k_visit3d(DevArgs a) {
             // time (plane_skip)
             const uint2* hs = a.hsb ? a.hsb + bd.slot_begin : nullptr;
             if (!plane_skip(TD, fminf(fminf(TA, TB), TC), slot_bound(hs, j, 3)))
-              nw[3] = fminf(TD, apex_update<3>(T, gm));
+              nw[3] = fminf(TD, apex_update(3, T, gm));
             if (!plane_skip(TA, fminf(fminf(TB, TD), TC), slot_bound(hs, j, 0)))
-              nw[0] = fminf(TA, apex_update<0>(T, gm));
+              nw[0] = fminf(TA, apex_update(0, T, gm));
             if (!plane_skip(TB, fminf(fminf(TA, TD), TC), slot_bound(hs, j, 1)))
-              nw[1] = fminf(TB, apex_update<1>(T, gm));
+              nw[1] = fminf(TB, apex_update(1, T, gm));
             if (!plane_skip(TC, fminf(fminf(TA, TB), TD), slot_bound(hs, j, 2)))
-              nw[2] = fminf(TC, apex_update<2>(T, gm));
+              nw[2] = fminf(TC, apex_update(2, T, gm));
           }
           if constexpr (kPrec) {
             // flagged tet: the four updates in FP64 from FP64 products
@@ -1001,10 +1001,10 @@ __device__ __forceinline__ bool check_pass(const DevArgs& a, const BlockDesc& bd
                                  s.coef[3 * pitch + j], s.coef[4 * pitch + j], s.coef[5 * pitch + j]);
     float u;
     switch (k) {
-      case 0: u = apex_update<0>(T, gm); break;
-      case 1: u = apex_update<1>(T, gm); break;
-      case 2: u = apex_update<2>(T, gm); break;
-      default: u = apex_update<3>(T, gm); break;
+      case 0: u = apex_update(0, T, gm); break;
+      case 1: u = apex_update(1, T, gm); break;
+      case 2: u = apex_update(2, T, gm); break;
+      default: u = apex_update(3, T, gm); break;
     }
     const float Tk = (k == 0) ? T[0] : (k == 1) ? T[1] : (k == 2) ? T[2] : T[3];
     // (double)(old - candidate) >= 1e-5 in the reference
@@ -1205,10 +1205,10 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a, int role) {
                                      s.coef[3 * pitch + j], s.coef[4 * pitch + j], s.coef[5 * pitch + j]);
         float u;
         switch (k) {
-          case 0: u = apex_update<0>(T, gm); break;
-          case 1: u = apex_update<1>(T, gm); break;
-          case 2: u = apex_update<2>(T, gm); break;
-          default: u = apex_update<3>(T, gm); break;
+          case 0: u = apex_update(0, T, gm); break;
+          case 1: u = apex_update(1, T, gm); break;
+          case 2: u = apex_update(2, T, gm); break;
+          default: u = apex_update(3, T, gm); break;
         }
         // T[k], id[k] by selects: a runtime index would put the arrays in local memory
         const float Tk = (k == 0) ? T[0] : (k == 1) ? T[1] : (k == 2) ? T[2] : T[3];
@@ -1254,6 +1254,109 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a, int role) {
       atomicAdd(&a.ctl->fim_halo, (unsigned long long)bd.nhalo);
       atomicAdd(&a.ctl->fim_owned, (unsigned long long)nown);
     }
+    __syncthreads();
+  }
+  stamp_end(a, iter, 0);
+}
+
+#include "visit3d.cuh"
+
+// ===========================================================================
+// 3D sweeps and checks of one iteration (the reference's two sweeps; k_sweep3d runs
+// other sweep counts).  CTAs claim the active blocks, then the check candidates queued
+// by the previous iteration's commit; a candidate that moves is appended to this
+// iteration's active list and swept in the same visit.
+// ===========================================================================
+__global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
+  pdl_begin();
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ __align__(8) unsigned long long bar;
+  __shared__ int s_item;
+  __shared__ int s_n[2];
+  __shared__ volatile int s_moved;
+  const SmemV s = carve_visit3d(sm, a);
+  const int tid = threadIdx.x, NT = blockDim.x;
+  Ctl* ctl = a.ctl;
+  const int iter = ctl->iter;
+  const int stamp = iter + 1;
+  const int nact = ctl->nact;
+  const int* cand = a.cand + (size_t)((iter + 1) & 1) * a.nb;
+  const int count = nact + ctl->ncand[(iter + 1) & 1];
+  int* list = act_list(a, iter);
+  stamp_start(a, iter, 0);
+  if (tid == 0) mbar_init(&bar, 1);
+  if (tid < 2) s_n[tid] = 0;
+  __syncthreads();
+  unsigned parity = 0;
+  // the first block of a CTA is its own index; later ones come from the counter
+  // (a CTA without a first block exits without touching it)
+  int item = blockIdx.x;
+  // a single instance's finished flag, read once (it changes only between launches):
+  // spares every visit the instance lookup
+  const int done1 = (a.ninst == 1) ? a.inst_done[0] : -1;
+  while (item < count) {
+    const bool chk = item >= nact;  // a check candidate
+    const int b = chk ? cand[item - nact] : list[item];
+    const BlockDesc bd = a.blocks[b];
+    // instance finished: leave its blocks alone; at its cap: its checks only
+    const int ist = done1 >= 0 ? done1 : a.inst_done[a.blk_inst[b]];
+    bool sweep = ist == 0;
+    if (ist != 1 && (sweep || chk)) {
+      if (!load_visit3d(a, bd, s, &bar, parity, chk ? a.chk_memo : a.fim_memo)) {
+        if (tid == 0) atomicOr(&a.ctl->error, kErrWait);
+        (void)mbar_wait(&bar, parity ^ 1u);
+        sweep = false;
+      } else {
+        __syncthreads();
+        const int nown = bd.nowned;
+        if (chk) {
+          const bool moved = check_visit3d(a, bd, s, s_n, &s_moved);
+          if (tid == 0) {  // the previous iteration's check (run_check_neghbor)
+            atomicAdd(&ctl->chk_visits, 1ull);
+            atomicAdd(&ctl->updates, (unsigned long long)nown);
+            count_visit(a, iter - 1, 1, bd.nslots, bd.nhalo, nown);
+            atomicAdd(&ctl->slot_visits, (unsigned long long)bd.nslots);
+            atomicAdd(&ctl->halo_visits, (unsigned long long)bd.nhalo);
+            atomicAdd(&ctl->owned_visits, (unsigned long long)nown);
+            if (moved && sweep) list[nact + atomicAdd(&ctl->nadd, 1)] = b;
+          }
+          sweep = sweep && moved;
+        }
+        if (sweep) {
+          sweep_visit3d(a, bd, s, s_n, chk);
+          int myconv = 1;
+          for (int k = tid; k < nown; k += NT) {
+            const float ov = __int_as_float(s.v1[k]), nv = __int_as_float(s.v2[k]);
+            float res = ov - nv;
+            if (res < 0.0f) res = -res;
+            myconv &= (res <= kEps3DLe) ? 1 : 0;
+            a.Tb[bd.vbase + k] = nv;
+          }
+          const int allc = __syncthreads_and(myconv);
+          if (tid == 0) {
+            a.conv[b] = allc;
+            if (!allc) a.stampA[b] = stamp;
+            atomicAdd(&a.inst_swept[a.blk_inst[b]], 1);
+            atomicAdd(&ctl->fim_visits, 1ull);
+            atomicAdd(&ctl->updates, 2ull * nown);
+            count_visit(a, iter, 0, bd.nslots, bd.nhalo, nown);
+            if (chk) {  // streamed once, with the check
+              count_visit(a, iter, 2, bd.nslots, bd.nhalo, nown);
+            } else {
+              atomicAdd(&ctl->slot_visits, (unsigned long long)bd.nslots);
+              atomicAdd(&ctl->halo_visits, (unsigned long long)bd.nhalo);
+              atomicAdd(&ctl->owned_visits, (unsigned long long)nown);
+            }
+            atomicAdd(&ctl->fim_slots, (unsigned long long)bd.nslots);
+            atomicAdd(&ctl->fim_halo, (unsigned long long)bd.nhalo);
+            atomicAdd(&ctl->fim_owned, (unsigned long long)nown);
+          }
+        }
+      }
+    }
+    if (tid == 0) s_item = (int)gridDim.x + atomicAdd(&ctl->work_a, 1);
+    __syncthreads();
+    item = s_item;
     __syncthreads();
   }
   stamp_end(a, iter, 0);
@@ -2320,10 +2423,10 @@ __global__ void k_selftest_tet_group(const float* in, float* out, int n) {
     const float T[4] = {a[0], a[1], a[2], a[3]};
     const TetGram g = tet_gram9(a[4], a[5], a[6], a[7], a[8], a[9]);
     float* o = out + 4 * (size_t)i;
-    o[0] = fminf(T[0], apex_update<0>(T, g));
-    o[1] = fminf(T[1], apex_update<1>(T, g));
-    o[2] = fminf(T[2], apex_update<2>(T, g));
-    o[3] = fminf(T[3], apex_update<3>(T, g));
+    o[0] = fminf(T[0], apex_update(0, T, g));
+    o[1] = fminf(T[1], apex_update(1, T, g));
+    o[2] = fminf(T[2], apex_update(2, T, g));
+    o[3] = fminf(T[3], apex_update(3, T, g));
   }
 }
 __global__ void k_selftest_tri(const float* in, float* out, int n) {
@@ -2765,8 +2868,16 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
         if (!P.prec && si + 64 <= (size_t)maxsm) vsmem = si;
         else if (!P.prec) kv_fim = (void*)k_visit3d<false>;
 #endif
+        // the reference's two sweeps have a kernel of their own
+        const size_t sv = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned);
+        if (!P.prec && sweeps == 2 && P.chk_memo && sv + 64 <= (size_t)maxsm) {
+          kv_fim = (void*)k_items3d;
+          vsmem = sv;
+          a.chk_memo = P.chk_memo;
+        }
 #if EIK_SWEEP_MEMO
-        if (kv_fim == (void*)k_sweep3d && P.chk_memo) a.fim_memo = P.chk_memo + P.coef_n / 6;
+        if ((kv_fim == (void*)k_sweep3d || kv_fim == (void*)k_items3d) && P.chk_memo)
+          a.fim_memo = P.chk_memo + P.coef_n / 6;
 #endif
 #if EIK_CHECK_ITEMS
         if (!P.prec && sc + 64 <= (size_t)maxsm) vsmem_chk = sc;
@@ -2775,7 +2886,7 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
         (void)si;
         (void)sc;
       }
-      a.fused = (EIK_FUSED_CHECK && kv_fim == (void*)k_sweep3d && kv_chk == (void*)k_check3d) ? 1 : 0;
+      a.fused = (kv_fim == (void*)k_items3d || (EIK_FUSED_CHECK && kv_fim == (void*)k_sweep3d && kv_chk == (void*)k_check3d)) ? 1 : 0;
     } else if (slot2d) {
       vthreads = std::max(32, (P.max_slots_pad + 31) & ~31);
       vsmem = vsmem_chk = smem_bytes_slot2d(P.max_slots_pad, P.max_local, P.max_owned);

@@ -213,10 +213,11 @@ __device__ __forceinline__ float tet_update(float TA, float TB, float TC, float 
 // a different kernel shape can round differently.  Here every product, sum,
 // quotient and square root is one IEEE operation (__fmul_rn, __fadd_rn, __fmaf_rn,
 // __fdiv_rn, __fsqrt_rn) that the compiler cannot fuse or split, so the result no
-// longer depends on the surrounding code, and a template mask states, for each sum
-// or difference of two products, which product the reference's kernel fuses: bit S
-// set = the second product is fused (x*y - z*w -> fma(-z, w, x*y)), clear = the
-// first (fma(x, y, -(z*w))).
+// longer depends on the surrounding code, and a mask states, for each sum or
+// difference of two products (a site, numbered 0..51 in the order of the
+// reference's statements), which product the reference's kernel fuses: bit S set =
+// the second product is fused (x*y - z*w -> fma(-z, w, x*y)), clear = the first
+// (fma(x, y, -(z*w))).
 //
 // The four masks below reproduce the reference kernel's own roundings for the four
 // apex updates of a slot: they were fitted to, and reproduce bit for bit, the
@@ -232,41 +233,40 @@ constexpr unsigned long long kFuseApexB = 0x6301902630000ull;  // B from A, D, C
 constexpr unsigned long long kFuseApexC = 0x4203182420002ull;  // C from A, B, D
 constexpr unsigned long long kFuseApexD = 0x0000001100000000ull;  // D from A, B, C
 
-// Sites in R take their choice from the runtime mask m instead of M (one body
-// serving several masks): the same two operations, operands picked by selects.
-template <unsigned long long M, unsigned long long R, int S>
-__device__ __forceinline__ float x_ms(unsigned long long m, float x, float y, float z, float w) {  // x*y - z*w
-  if constexpr (((R >> S) & 1ull) != 0) {
-    const bool b = ((m >> S) & 1ull) != 0;
-    const float pr = __fmul_rn(b ? x : z, b ? y : w);
-    return __fmaf_rn(b ? -z : x, b ? w : y, b ? pr : -pr);
-  } else if constexpr (((M >> S) & 1ull) != 0) {
-    return __fmaf_rn(-z, w, __fmul_rn(x, y));
-  } else {
-    return __fmaf_rn(x, y, -__fmul_rn(z, w));
-  }
+// The masks agree at most sites; the others follow three flags of the apex kind:
+// ab (A and B), abc (A, B and C), c (C alone).
+struct ApexFuse {
+  bool ab, abc, c;
+};
+constexpr unsigned long long fuse_mask(ApexFuse f) {
+  const unsigned long long one = 1ull;
+  return (one << 32 | one << 36) |
+         (f.ab ? (one << 16 | one << 21 | one << 35 | one << 44 | one << 49) : 0ull) |
+         (f.abc ? (one << 17 | one << 22 | one << 25 | one << 45 | one << 50) : 0ull) |
+         (f.c ? (one << 1 | one << 31 | one << 37) : 0ull);
 }
-template <unsigned long long M, unsigned long long R, int S>
-__device__ __forceinline__ float x_ma(unsigned long long m, float x, float y, float z, float w) {  // x*y + z*w
-  if constexpr (((R >> S) & 1ull) != 0) {
-    const bool b = ((m >> S) & 1ull) != 0;
-    const float pr = __fmul_rn(b ? x : z, b ? y : w);
-    return __fmaf_rn(b ? z : x, b ? w : y, pr);
-  } else if constexpr (((M >> S) & 1ull) != 0) {
-    return __fmaf_rn(z, w, __fmul_rn(x, y));
-  } else {
-    return __fmaf_rn(x, y, __fmul_rn(z, w));
-  }
+__host__ __device__ constexpr ApexFuse apex_fuse(int k) { return ApexFuse{k < 2, k < 3, k == 2}; }
+static_assert(fuse_mask(apex_fuse(0)) == kFuseApexA && fuse_mask(apex_fuse(1)) == kFuseApexB &&
+                  fuse_mask(apex_fuse(2)) == kFuseApexC && fuse_mask(apex_fuse(3)) == kFuseApexD,
+              "the flags must give the fitted masks");
+
+// x*y - z*w and x*y + z*w with the second (b) or the first product fused
+__device__ __forceinline__ float x_ms(bool b, float x, float y, float z, float w) {
+  const float pr = __fmul_rn(b ? x : z, b ? y : w);
+  return __fmaf_rn(b ? -z : x, b ? w : y, b ? pr : -pr);
+}
+__device__ __forceinline__ float x_ma(bool b, float x, float y, float z, float w) {
+  const float pr = __fmul_rn(b ? x : z, b ? y : w);
+  return __fmaf_rn(b ? z : x, b ? w : y, pr);
 }
 // (l1*XX + l2*XY + XZ)*l1 + (l1*XY + l2*YY + YZ)*l2 + (l1*XZ + l2*YZ + ZZ): the metric
-// length of the path from the apex to the point l1 A + l2 B + l3 C (sites S..S+3)
-template <unsigned long long M, unsigned long long R, int S>
-__device__ __forceinline__ float x_dist3(unsigned long long m, float l1, float l2, float ACAC, float ACBC,
-                                         float ACCD, float BCBC, float BCCD, float CDCD) {
-  const float X = __fadd_rn(x_ma<M, R, S>(m, l1, ACAC, l2, ACBC), ACCD);
-  const float Y = __fadd_rn(x_ma<M, R, S + 1>(m, l1, ACBC, l2, BCBC), BCCD);
-  const float Z = __fadd_rn(x_ma<M, R, S + 2>(m, l1, ACCD, l2, BCCD), CDCD);
-  return __fadd_rn(x_ma<M, R, S + 3>(m, X, l1, Y, l2), Z);
+// length of the path from the apex to the point l1 A + l2 B + l3 C
+__device__ __forceinline__ float x_dist3(ApexFuse f, float l1, float l2, float ACAC, float ACBC, float ACCD,
+                                         float BCBC, float BCCD, float CDCD) {
+  const float X = __fadd_rn(__fmaf_rn(l1, ACAC, __fmul_rn(l2, ACBC)), ACCD);
+  const float Y = __fadd_rn(x_ma(f.ab, l1, ACBC, l2, BCBC), BCCD);
+  const float Z = __fadd_rn(x_ma(f.abc, l1, ACCD, l2, BCCD), CDCD);
+  return __fadd_rn(__fmaf_rn(X, l1, __fmul_rn(Y, l2)), Z);
 }
 // (l*XX + XY)*l + (l*XY + YY): the same on an edge
 __device__ __forceinline__ float x_dist2(float l, float XX, float XY, float YY) {
@@ -277,344 +277,128 @@ __device__ __forceinline__ float x_root(float num, float p) {
   return root_quot_slow(num, p);
 }
 
-// localSolverTet1 (CUDA_kernels.cu:69-225) with the roundings of mask M: the update
-// of apex D from A, B, C; the candidate order and every expression tree are the
-// reference's.
-template <unsigned long long M, unsigned long long R = 0>
-__device__ __forceinline__ float tet_update_x(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                              float BCBC, float BCCD, float CDCD, unsigned long long m = 0) {
-  if (TA >= kLarge3DDev && TB >= kLarge3DDev && TC >= kLarge3DDev) return kLarge3DDev;
-  float p, q, r, l1, l2, l3, delta;
-  float fBC = kLarge3DDev, fAB = kLarge3DDev, fAC = kLarge3DDev, TD = kLarge3DDev;
-  const float TAC = __fsub_rn(TC, TA), TBC = __fsub_rn(TC, TB), TAB = __fsub_rn(TB, TA);
-  // ---- face BC (lambda1 = 0) ----
-  p = x_ms<M, R, 0>(m, __fmul_rn(BCBC, TBC), TBC, BCBC, BCBC);
-  q = x_ms<M, R, 1>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TBC), TBC, __fmul_rn(2.0f, BCBC), BCCD);
-  r = x_ms<M, R, 2>(m, __fmul_rn(TBC, TBC), CDCD, BCCD, BCCD);
-  delta = x_ms<M, R, 3>(m, q, q, __fmul_rn(4.0f, p), r);
+// localSolverTet1 (CUDA_kernels.cu:69-225) takes the least of the candidates on the
+// face's edges BC, AB and AC and inside the face ABC.  A minimum does not depend on its
+// order (a NaN candidate is ignored wherever it stands), so the update is written as one
+// function per edge and one for the inside, each starting from LARGENUM as the
+// reference's candidates do.
+
+// Edge XC, X = B or A: sites 0-5 (BC) and 24-29 (AC).  AC's second candidate keeps a
+// zero-weight TB term in the reference, which leaves TA*l1 rounded by itself; its sum
+// is then the one with the second product fused.
+__device__ __forceinline__ float tet_part_edge(bool ac, ApexFuse f, float TX, float TC, float XX, float XC, float CC) {
+  const float T = __fsub_rn(TC, TX);
+  const float p = __fmaf_rn(__fmul_rn(XX, T), T, -__fmul_rn(XX, XX));
+  const float q = x_ms(ac ? f.abc : f.c, __fmul_rn(__fadd_rn(XC, XC), T), T, __fmul_rn(2.0f, XX), XC);
+  const float r = __fmaf_rn(__fmul_rn(T, T), CC, -__fmul_rn(XC, XC));
+  const float delta = __fmaf_rn(q, q, -__fmul_rn(__fmul_rn(4.0f, p), r));
+  float best = fminf(__fadd_rn(TX, __fsqrt_rn(__fadd_rn(__fadd_rn(XX, XC), __fadd_rn(XC, CC)))),
+                     __fadd_rn(TC, __fsqrt_rn(CC)));
+  best = fminf(kLarge3DDev, best);
   if (delta >= 0.0f) {
     const float sd = __fsqrt_rn(delta);
-    l2 = x_root(__fadd_rn(-q, sd), p);
-    l3 = __fsub_rn(1.0f, l2);
-    if (l2 >= 0 && l2 <= 1)
-      fBC = fminf(fBC, __fadd_rn(x_ma<M, R, 4>(m, TB, l2, TC, l3), __fsqrt_rn(x_dist2(l2, BCBC, BCCD, CDCD))));
-    l2 = x_root(__fsub_rn(-q, sd), p);
-    l3 = __fsub_rn(1.0f, l2);
-    if (l2 >= 0 && l2 <= 1)
-      fBC = fminf(fBC, __fadd_rn(x_ma<M, R, 5>(m, TB, l2, TC, l3), __fsqrt_rn(x_dist2(l2, BCBC, BCCD, CDCD))));
+    float l = x_root(__fadd_rn(-q, sd), p);
+    float m = __fsub_rn(1.0f, l);
+    if (l >= 0 && l <= 1)
+      best = fminf(best, __fadd_rn(__fmaf_rn(TX, l, __fmul_rn(TC, m)), __fsqrt_rn(x_dist2(l, XX, XC, CC))));
+    l = x_root(__fsub_rn(-q, sd), p);
+    m = __fsub_rn(1.0f, l);
+    if (l >= 0 && l <= 1)
+      best = fminf(best, __fadd_rn(x_ma(ac, TX, l, TC, m), __fsqrt_rn(x_dist2(l, XX, XC, CC))));
   }
-  const float eB = __fadd_rn(TB, __fsqrt_rn(__fadd_rn(__fadd_rn(BCBC, BCCD), __fadd_rn(BCCD, CDCD))));
-  const float eC = __fadd_rn(TC, __fsqrt_rn(CDCD));
-  fBC = fminf(fBC, fminf(eB, eC));
-  // ---- face AB (lambda3 = 0) ----
+  return best;
+}
+// Edge AB (sites 6-23); its end points are candidates of the other two edges.
+__device__ __forceinline__ float tet_part_ab(ApexFuse f, float TA, float TB, float ACAC, float ACBC, float ACCD,
+                                             float BCBC, float BCCD, float CDCD) {
+  const float TAB = __fsub_rn(TB, TA);
   const float gx = __fsub_rn(ACAC, ACBC), gy = __fsub_rn(ACBC, BCBC), gz = __fsub_rn(ACCD, BCCD);
   const float TAB2 = __fmul_rn(TAB, TAB);
-  const float P1 = x_ms<M, R, 6>(m, TAB2, ACAC, gx, gx);
-  const float P2 = x_ms<M, R, 7>(m, __fmul_rn(BCBC, TAB), TAB, gy, gy);
-  const float P3 = x_ms<M, R, 8>(m, __fmul_rn(__fadd_rn(ACBC, ACBC), TAB), TAB, __fmul_rn(2.0f, gx), gy);
-  p = __fsub_rn(__fadd_rn(P1, P2), P3);
-  const float P4 = x_ms<M, R, 9>(m, __fmul_rn(__fadd_rn(ACCD, ACCD), TAB), TAB, __fmul_rn(2.0f, gx), gz);
-  const float P5 = x_ms<M, R, 10>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TAB), TAB, __fmul_rn(2.0f, gy), gz);
-  q = __fsub_rn(__fadd_rn(__fadd_rn(__fmul_rn(-P2, 2.0f), P3), P4), P5);
-  r = __fadd_rn(__fadd_rn(x_ms<M, R, 11>(m, TAB2, BCBC, gy, gy), P5), x_ms<M, R, 12>(m, TAB2, CDCD, gz, gz));
-  delta = x_ms<M, R, 13>(m, q, q, __fmul_rn(4.0f, p), r);
-  if (delta >= 0.0f) {
-    const float sd = __fsqrt_rn(delta);
-    l1 = x_root(__fadd_rn(-q, sd), p);
-    l2 = __fsub_rn(1.0f, l1);
-    if (l1 >= 0 && l1 <= 1)
-      fAB = fminf(fAB, __fadd_rn(x_ma<M, R, 14>(m, TA, l1, TB, l2),
-                                 __fsqrt_rn(x_dist3<M, R, 15>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-    l1 = x_root(__fsub_rn(-q, sd), p);
-    l2 = __fsub_rn(1.0f, l1);
-    if (l1 >= 0 && l1 <= 1)
-      fAB = fminf(fAB, __fadd_rn(x_ma<M, R, 19>(m, TA, l1, TB, l2),
-                                 __fsqrt_rn(x_dist3<M, R, 20>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-  }
-  const float eA = __fadd_rn(TA, __fsqrt_rn(__fadd_rn(__fadd_rn(ACAC, ACCD), __fadd_rn(ACCD, CDCD))));
-  fAB = fminf(fAB, fminf(eB, eA));
-  // ---- face AC (lambda2 = 0) ----
-  const float TAC2 = __fmul_rn(TAC, TAC);
-  p = x_ms<M, R, 24>(m, __fmul_rn(ACAC, TAC), TAC, ACAC, ACAC);
-  const float qAC = x_ms<M, R, 25>(m, __fmul_rn(__fadd_rn(ACCD, ACCD), TAC), TAC, __fmul_rn(2.0f, ACAC), ACCD);
-  const float rAC = x_ms<M, R, 26>(m, TAC2, CDCD, ACCD, ACCD);
-  delta = x_ms<M, R, 27>(m, qAC, qAC, __fmul_rn(4.0f, p), rAC);
-  if (delta >= 0.0f) {
-    const float sd = __fsqrt_rn(delta);
-    l1 = x_root(__fadd_rn(-qAC, sd), p);
-    l3 = __fsub_rn(1.0f, l1);
-    if (l1 >= 0 && l1 <= 1)
-      fAC = fminf(fAC, __fadd_rn(x_ma<M, R, 28>(m, TA, l1, TC, l3), __fsqrt_rn(x_dist2(l1, ACAC, ACCD, CDCD))));
-    l1 = x_root(__fsub_rn(-qAC, sd), p);
-    l3 = __fsub_rn(1.0f, l1);
-    // the second candidate keeps a zero-weight TB term, as the reference does
-    if (l1 >= 0 && l1 <= 1)
-      fAC = fminf(fAC, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 29>(m, TA, l1, TB, 0.0f)),
-                                 __fsqrt_rn(x_dist2(l1, ACAC, ACCD, CDCD))));
-  }
-  fAC = fminf(fAC, fminf(eA, eC));
-  // ---- inside face ABC: lambda2 = (s*lambda1 + t)/(h + 1e-8) ----
-  const float s = x_ms<M, R, 30>(m, TAC, ACBC, TBC, ACAC);
-  const float t = x_ms<M, R, 31>(m, TAC, BCCD, TBC, ACCD);
-  const float h = -x_ms<M, R, 32>(m, TAC, BCBC, TBC, ACBC);
-  const float A1 = x_ms<M, R, 33>(m, TAC2, ACAC, ACAC, ACAC);
-  const float A2 = x_ms<M, R, 34>(m, __fmul_rn(BCBC, TAC), TAC, ACBC, ACBC);
-  const float A3 = x_ms<M, R, 35>(m, __fmul_rn(__fadd_rn(ACBC, ACBC), TAC), TAC, __fmul_rn(2.0f, ACAC), ACBC);
-  const float A4 = x_ms<M, R, 37>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TAC), TAC, __fmul_rn(2.0f, ACBC), ACCD);
-  p = __fmaf_rn(__fmul_rn(A3, s), h, x_ma<M, R, 36>(m, __fmul_rn(A1, h), h, __fmul_rn(A2, s), s));
-  q = __fmaf_rn(__fmul_rn(A4, s), h,
-                __fmaf_rn(__fmul_rn(qAC, h), h, x_ma<M, R, 38>(m, __fmul_rn(__fmul_rn(A2, 2.0f), s), t, __fmul_rn(A3, t), h)));
-  r = __fmaf_rn(__fmul_rn(rAC, h), h, x_ma<M, R, 40>(m, __fmul_rn(x_ms<M, R, 39>(m, TAC2, BCBC, ACBC, ACBC), t), t,
-                                                   __fmul_rn(A4, t), h));
-  delta = x_ms<M, R, 41>(m, q, q, __fmul_rn(4.0f, p), r);
-  if (delta >= 0.0f) {
-    const float sd = __fsqrt_rn(delta);
-    l1 = x_root(__fadd_rn(-q, sd), p);
-    l2 = small_quot(__fmaf_rn(s, l1, t), h);
-    l3 = __fsub_rn(__fsub_rn(1.0f, l1), l2);
-    if (l1 >= 0 && l1 <= 1 && l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)
-      TD = fminf(TD, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 42>(m, TA, l1, TB, l2)),
-                               __fsqrt_rn(x_dist3<M, R, 43>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-    l1 = x_root(__fsub_rn(-q, sd), p);
-    l2 = small_quot(__fmaf_rn(s, l1, t), h);
-    l3 = __fsub_rn(__fsub_rn(1.0f, l1), l2);
-    if (l1 >= 0 && l1 <= 1 && l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)
-      TD = fminf(TD, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 47>(m, TA, l1, TB, l2)),
-                               __fsqrt_rn(x_dist3<M, R, 48>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-  }
-  return fminf(TD, fminf(fBC, fminf(fAB, fAC)));
-}
-
-// The same update with the edge-face candidates (faces BC, AB, AC) evaluated
-// without branches: both roots of each face are computed whatever the
-// discriminant's sign, and a candidate enters the minimum only where the branching
-// form would have taken it (a negative discriminant gives NaN roots, which fail
-// the [0, 1] tests).  Every value is the explicitly rounded one of tet_update_x and
-// the minimum does not depend on the order of its operands, so the result is the
-// same bits; the interior face keeps its branch (its second quotient has a slow
-// path that a NaN input would take).
-template <unsigned long long M, unsigned long long R = 0>
-__device__ __forceinline__ float tet_update_xb(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                               float BCBC, float BCCD, float CDCD, unsigned long long m = 0) {
-  if (TA >= kLarge3DDev && TB >= kLarge3DDev && TC >= kLarge3DDev) return kLarge3DDev;
-  const float L = kLarge3DDev;
-  const float TAC = __fsub_rn(TC, TA), TBC = __fsub_rn(TC, TB), TAB = __fsub_rn(TB, TA);
-  // ---- face BC (lambda1 = 0) ----
-  float fBC;
-  {
-    const float p = x_ms<M, R, 0>(m, __fmul_rn(BCBC, TBC), TBC, BCBC, BCBC);
-    const float q = x_ms<M, R, 1>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TBC), TBC, __fmul_rn(2.0f, BCBC), BCCD);
-    const float r = x_ms<M, R, 2>(m, __fmul_rn(TBC, TBC), CDCD, BCCD, BCCD);
-    const float delta = x_ms<M, R, 3>(m, q, q, __fmul_rn(4.0f, p), r);
-    const bool ok = delta >= 0.0f;
-    const float sd = __fsqrt_rn(delta);
-    const float a2 = x_root(__fadd_rn(-q, sd), p), a3 = __fsub_rn(1.0f, a2);
-    const float b2 = x_root(__fsub_rn(-q, sd), p), b3 = __fsub_rn(1.0f, b2);
-    const float ca = __fadd_rn(x_ma<M, R, 4>(m, TB, a2, TC, a3), __fsqrt_rn(x_dist2(a2, BCBC, BCCD, CDCD)));
-    const float cb = __fadd_rn(x_ma<M, R, 5>(m, TB, b2, TC, b3), __fsqrt_rn(x_dist2(b2, BCBC, BCCD, CDCD)));
-    // seeded with LARGENUM as the branching form (a NaN candidate is ignored)
-    fBC = fminf(fminf(L, (ok && a2 >= 0 && a2 <= 1) ? ca : L), (ok && b2 >= 0 && b2 <= 1) ? cb : L);
-  }
-  const float eB = __fadd_rn(TB, __fsqrt_rn(__fadd_rn(__fadd_rn(BCBC, BCCD), __fadd_rn(BCCD, CDCD))));
-  const float eC = __fadd_rn(TC, __fsqrt_rn(CDCD));
-  const float eA = __fadd_rn(TA, __fsqrt_rn(__fadd_rn(__fadd_rn(ACAC, ACCD), __fadd_rn(ACCD, CDCD))));
-  // ---- face AB (lambda3 = 0) ----
-  float fAB;
-  {
-    const float gx = __fsub_rn(ACAC, ACBC), gy = __fsub_rn(ACBC, BCBC), gz = __fsub_rn(ACCD, BCCD);
-    const float TAB2 = __fmul_rn(TAB, TAB);
-    const float P1 = x_ms<M, R, 6>(m, TAB2, ACAC, gx, gx);
-    const float P2 = x_ms<M, R, 7>(m, __fmul_rn(BCBC, TAB), TAB, gy, gy);
-    const float P3 = x_ms<M, R, 8>(m, __fmul_rn(__fadd_rn(ACBC, ACBC), TAB), TAB, __fmul_rn(2.0f, gx), gy);
-    const float p = __fsub_rn(__fadd_rn(P1, P2), P3);
-    const float P4 = x_ms<M, R, 9>(m, __fmul_rn(__fadd_rn(ACCD, ACCD), TAB), TAB, __fmul_rn(2.0f, gx), gz);
-    const float P5 = x_ms<M, R, 10>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TAB), TAB, __fmul_rn(2.0f, gy), gz);
-    const float q = __fsub_rn(__fadd_rn(__fadd_rn(__fmul_rn(-P2, 2.0f), P3), P4), P5);
-    const float r = __fadd_rn(__fadd_rn(x_ms<M, R, 11>(m, TAB2, BCBC, gy, gy), P5), x_ms<M, R, 12>(m, TAB2, CDCD, gz, gz));
-    const float delta = x_ms<M, R, 13>(m, q, q, __fmul_rn(4.0f, p), r);
-    const bool ok = delta >= 0.0f;
-    const float sd = __fsqrt_rn(delta);
-    const float a1 = x_root(__fadd_rn(-q, sd), p), a2 = __fsub_rn(1.0f, a1);
-    const float b1 = x_root(__fsub_rn(-q, sd), p), b2 = __fsub_rn(1.0f, b1);
-    const float ca = __fadd_rn(x_ma<M, R, 14>(m, TA, a1, TB, a2),
-                               __fsqrt_rn(x_dist3<M, R, 15>(m, a1, a2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD)));
-    const float cb = __fadd_rn(x_ma<M, R, 19>(m, TA, b1, TB, b2),
-                               __fsqrt_rn(x_dist3<M, R, 20>(m, b1, b2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD)));
-    // seeded with LARGENUM as the branching form (a NaN candidate is ignored)
-    fAB = fminf(fminf(L, (ok && a1 >= 0 && a1 <= 1) ? ca : L), (ok && b1 >= 0 && b1 <= 1) ? cb : L);
-  }
-  // ---- face AC (lambda2 = 0) ----
-  const float TAC2 = __fmul_rn(TAC, TAC);
-  const float qAC = x_ms<M, R, 25>(m, __fmul_rn(__fadd_rn(ACCD, ACCD), TAC), TAC, __fmul_rn(2.0f, ACAC), ACCD);
-  const float rAC = x_ms<M, R, 26>(m, TAC2, CDCD, ACCD, ACCD);
-  float fAC;
-  {
-    const float p = x_ms<M, R, 24>(m, __fmul_rn(ACAC, TAC), TAC, ACAC, ACAC);
-    const float delta = x_ms<M, R, 27>(m, qAC, qAC, __fmul_rn(4.0f, p), rAC);
-    const bool ok = delta >= 0.0f;
-    const float sd = __fsqrt_rn(delta);
-    const float a1 = x_root(__fadd_rn(-qAC, sd), p), a3 = __fsub_rn(1.0f, a1);
-    const float b1 = x_root(__fsub_rn(-qAC, sd), p), b3 = __fsub_rn(1.0f, b1);
-    const float ca = __fadd_rn(x_ma<M, R, 28>(m, TA, a1, TC, a3), __fsqrt_rn(x_dist2(a1, ACAC, ACCD, CDCD)));
-    // the second candidate keeps a zero-weight TB term, as the reference does
-    const float cb = __fadd_rn(__fmaf_rn(TC, b3, x_ma<M, R, 29>(m, TA, b1, TB, 0.0f)),
-                               __fsqrt_rn(x_dist2(b1, ACAC, ACCD, CDCD)));
-    // seeded with LARGENUM as the branching form (a NaN candidate is ignored)
-    fAC = fminf(fminf(L, (ok && a1 >= 0 && a1 <= 1) ? ca : L), (ok && b1 >= 0 && b1 <= 1) ? cb : L);
-  }
-  const float edges = fminf(fminf(fBC, fminf(eB, eC)), fminf(fminf(fAB, fminf(eB, eA)), fminf(fAC, fminf(eA, eC))));
-  // ---- inside face ABC: lambda2 = (s*lambda1 + t)/(h + 1e-8) ----
-  const float s = x_ms<M, R, 30>(m, TAC, ACBC, TBC, ACAC);
-  const float t = x_ms<M, R, 31>(m, TAC, BCCD, TBC, ACCD);
-  const float h = -x_ms<M, R, 32>(m, TAC, BCBC, TBC, ACBC);
-  const float A1 = x_ms<M, R, 33>(m, TAC2, ACAC, ACAC, ACAC);
-  const float A2 = x_ms<M, R, 34>(m, __fmul_rn(BCBC, TAC), TAC, ACBC, ACBC);
-  const float A3 = x_ms<M, R, 35>(m, __fmul_rn(__fadd_rn(ACBC, ACBC), TAC), TAC, __fmul_rn(2.0f, ACAC), ACBC);
-  const float A4 = x_ms<M, R, 37>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TAC), TAC, __fmul_rn(2.0f, ACBC), ACCD);
-  const float p = __fmaf_rn(__fmul_rn(A3, s), h, x_ma<M, R, 36>(m, __fmul_rn(A1, h), h, __fmul_rn(A2, s), s));
-  const float q = __fmaf_rn(__fmul_rn(A4, s), h,
-                            __fmaf_rn(__fmul_rn(qAC, h), h,
-                                      x_ma<M, R, 38>(m, __fmul_rn(__fmul_rn(A2, 2.0f), s), t, __fmul_rn(A3, t), h)));
-  const float r = __fmaf_rn(__fmul_rn(rAC, h), h, x_ma<M, R, 40>(m, __fmul_rn(x_ms<M, R, 39>(m, TAC2, BCBC, ACBC, ACBC), t), t,
-                                                               __fmul_rn(A4, t), h));
-  const float delta = x_ms<M, R, 41>(m, q, q, __fmul_rn(4.0f, p), r);
-  float TD = L;
+  const float P1 = __fmaf_rn(TAB2, ACAC, -__fmul_rn(gx, gx));
+  const float P2 = __fmaf_rn(__fmul_rn(BCBC, TAB), TAB, -__fmul_rn(gy, gy));
+  const float P3 = __fmaf_rn(__fmul_rn(__fadd_rn(ACBC, ACBC), TAB), TAB, -__fmul_rn(__fmul_rn(2.0f, gx), gy));
+  const float p = __fsub_rn(__fadd_rn(P1, P2), P3);
+  const float P4 = __fmaf_rn(__fmul_rn(__fadd_rn(ACCD, ACCD), TAB), TAB, -__fmul_rn(__fmul_rn(2.0f, gx), gz));
+  const float P5 = __fmaf_rn(__fmul_rn(__fadd_rn(BCCD, BCCD), TAB), TAB, -__fmul_rn(__fmul_rn(2.0f, gy), gz));
+  const float q = __fsub_rn(__fadd_rn(__fadd_rn(__fmul_rn(-P2, 2.0f), P3), P4), P5);
+  const float r = __fadd_rn(__fadd_rn(__fmaf_rn(TAB2, BCBC, -__fmul_rn(gy, gy)), P5),
+                            __fmaf_rn(TAB2, CDCD, -__fmul_rn(gz, gz)));
+  const float delta = __fmaf_rn(q, q, -__fmul_rn(__fmul_rn(4.0f, p), r));
+  float best = kLarge3DDev;
   if (delta >= 0.0f) {
     const float sd = __fsqrt_rn(delta);
     float l1 = x_root(__fadd_rn(-q, sd), p);
-    float l2 = small_quot(__fmaf_rn(s, l1, t), h);
-    float l3 = __fsub_rn(__fsub_rn(1.0f, l1), l2);
-    if (l1 >= 0 && l1 <= 1 && l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)
-      TD = fminf(TD, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 42>(m, TA, l1, TB, l2)),
-                               __fsqrt_rn(x_dist3<M, R, 43>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
+    float l2 = __fsub_rn(1.0f, l1);
+    if (l1 >= 0 && l1 <= 1)
+      best = fminf(best, __fadd_rn(__fmaf_rn(TA, l1, __fmul_rn(TB, l2)),
+                                   __fsqrt_rn(x_dist3(f, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
     l1 = x_root(__fsub_rn(-q, sd), p);
-    l2 = small_quot(__fmaf_rn(s, l1, t), h);
-    l3 = __fsub_rn(__fsub_rn(1.0f, l1), l2);
-    if (l1 >= 0 && l1 <= 1 && l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)
-      TD = fminf(TD, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 47>(m, TA, l1, TB, l2)),
-                               __fsqrt_rn(x_dist3<M, R, 48>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
+    l2 = __fsub_rn(1.0f, l1);
+    if (l1 >= 0 && l1 <= 1)
+      best = fminf(best, __fadd_rn(__fmaf_rn(TA, l1, __fmul_rn(TB, l2)),
+                                   __fsqrt_rn(x_dist3(f, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
   }
-  return fminf(TD, edges);
+  return best;
 }
-
-// tet_update_x with the four faces' quadratic coefficients and discriminants
-// formed before any root is taken: the four chains are independent and can
-// interleave; the roots keep their branches.  Same operations, same bits.
-template <unsigned long long M, unsigned long long R = 0>
-__device__ __forceinline__ float tet_update_xd(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                               float BCBC, float BCCD, float CDCD, unsigned long long m = 0) {
-  if (TA >= kLarge3DDev && TB >= kLarge3DDev && TC >= kLarge3DDev) return kLarge3DDev;
-  const float L = kLarge3DDev;
-  const float TAC = __fsub_rn(TC, TA), TBC = __fsub_rn(TC, TB), TAB = __fsub_rn(TB, TA);
-  // face BC
-  const float pBC = x_ms<M, R, 0>(m, __fmul_rn(BCBC, TBC), TBC, BCBC, BCBC);
-  const float qBC = x_ms<M, R, 1>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TBC), TBC, __fmul_rn(2.0f, BCBC), BCCD);
-  const float rBC = x_ms<M, R, 2>(m, __fmul_rn(TBC, TBC), CDCD, BCCD, BCCD);
-  const float dBC = x_ms<M, R, 3>(m, qBC, qBC, __fmul_rn(4.0f, pBC), rBC);
-  // face AB
-  const float gx = __fsub_rn(ACAC, ACBC), gy = __fsub_rn(ACBC, BCBC), gz = __fsub_rn(ACCD, BCCD);
-  const float TAB2 = __fmul_rn(TAB, TAB);
-  const float P2 = x_ms<M, R, 7>(m, __fmul_rn(BCBC, TAB), TAB, gy, gy);
-  const float P3 = x_ms<M, R, 8>(m, __fmul_rn(__fadd_rn(ACBC, ACBC), TAB), TAB, __fmul_rn(2.0f, gx), gy);
-  const float pAB = __fsub_rn(__fadd_rn(x_ms<M, R, 6>(m, TAB2, ACAC, gx, gx), P2), P3);
-  const float P5 = x_ms<M, R, 10>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TAB), TAB, __fmul_rn(2.0f, gy), gz);
-  const float qAB = __fsub_rn(__fadd_rn(__fadd_rn(__fmul_rn(-P2, 2.0f), P3),
-                                        x_ms<M, R, 9>(m, __fmul_rn(__fadd_rn(ACCD, ACCD), TAB), TAB, __fmul_rn(2.0f, gx), gz)),
-                              P5);
-  const float rAB = __fadd_rn(__fadd_rn(x_ms<M, R, 11>(m, TAB2, BCBC, gy, gy), P5), x_ms<M, R, 12>(m, TAB2, CDCD, gz, gz));
-  const float dAB = x_ms<M, R, 13>(m, qAB, qAB, __fmul_rn(4.0f, pAB), rAB);
-  // face AC
+// Inside the face ABC, lambda2 = (s*lambda1 + t)/(h + 1e-8) (sites 30-51): the
+// candidate of the quadratic's root with +sqrt (minus = false) or -sqrt.
+struct TetInner {
+  float p, q, s, t, h, sd;  // sd < 0: no real root
+};
+__device__ __forceinline__ TetInner tet_inner_setup(ApexFuse f, float TA, float TB, float TC, float ACAC, float ACBC,
+                                                    float ACCD, float BCBC, float BCCD, float CDCD) {
+  TetInner o;
+  const float TAC = __fsub_rn(TC, TA), TBC = __fsub_rn(TC, TB);
   const float TAC2 = __fmul_rn(TAC, TAC);
-  const float pAC = x_ms<M, R, 24>(m, __fmul_rn(ACAC, TAC), TAC, ACAC, ACAC);
-  const float qAC = x_ms<M, R, 25>(m, __fmul_rn(__fadd_rn(ACCD, ACCD), TAC), TAC, __fmul_rn(2.0f, ACAC), ACCD);
-  const float rAC = x_ms<M, R, 26>(m, TAC2, CDCD, ACCD, ACCD);
-  const float dAC = x_ms<M, R, 27>(m, qAC, qAC, __fmul_rn(4.0f, pAC), rAC);
-  // face ABC
-  const float s = x_ms<M, R, 30>(m, TAC, ACBC, TBC, ACAC);
-  const float t = x_ms<M, R, 31>(m, TAC, BCCD, TBC, ACCD);
-  const float h = -x_ms<M, R, 32>(m, TAC, BCBC, TBC, ACBC);
-  const float A1 = x_ms<M, R, 33>(m, TAC2, ACAC, ACAC, ACAC);
-  const float A2 = x_ms<M, R, 34>(m, __fmul_rn(BCBC, TAC), TAC, ACBC, ACBC);
-  const float A3 = x_ms<M, R, 35>(m, __fmul_rn(__fadd_rn(ACBC, ACBC), TAC), TAC, __fmul_rn(2.0f, ACAC), ACBC);
-  const float A4 = x_ms<M, R, 37>(m, __fmul_rn(__fadd_rn(BCCD, BCCD), TAC), TAC, __fmul_rn(2.0f, ACBC), ACCD);
-  const float p = __fmaf_rn(__fmul_rn(A3, s), h, x_ma<M, R, 36>(m, __fmul_rn(A1, h), h, __fmul_rn(A2, s), s));
-  const float q = __fmaf_rn(__fmul_rn(A4, s), h,
-                            __fmaf_rn(__fmul_rn(qAC, h), h,
-                                      x_ma<M, R, 38>(m, __fmul_rn(__fmul_rn(A2, 2.0f), s), t, __fmul_rn(A3, t), h)));
-  const float r = __fmaf_rn(__fmul_rn(rAC, h), h, x_ma<M, R, 40>(m, __fmul_rn(x_ms<M, R, 39>(m, TAC2, BCBC, ACBC, ACBC), t), t,
-                                                               __fmul_rn(A4, t), h));
-  const float delta = x_ms<M, R, 41>(m, q, q, __fmul_rn(4.0f, p), r);
-  const float eB = __fadd_rn(TB, __fsqrt_rn(__fadd_rn(__fadd_rn(BCBC, BCCD), __fadd_rn(BCCD, CDCD))));
-  const float eC = __fadd_rn(TC, __fsqrt_rn(CDCD));
-  const float eA = __fadd_rn(TA, __fsqrt_rn(__fadd_rn(__fadd_rn(ACAC, ACCD), __fadd_rn(ACCD, CDCD))));
-  float fBC = L, fAB = L, fAC = L, TD = L, l1, l2, l3;
-  if (dBC >= 0.0f) {
-    const float sd = __fsqrt_rn(dBC);
-    l2 = x_root(__fadd_rn(-qBC, sd), pBC);
-    l3 = __fsub_rn(1.0f, l2);
-    if (l2 >= 0 && l2 <= 1)
-      fBC = fminf(fBC, __fadd_rn(x_ma<M, R, 4>(m, TB, l2, TC, l3), __fsqrt_rn(x_dist2(l2, BCBC, BCCD, CDCD))));
-    l2 = x_root(__fsub_rn(-qBC, sd), pBC);
-    l3 = __fsub_rn(1.0f, l2);
-    if (l2 >= 0 && l2 <= 1)
-      fBC = fminf(fBC, __fadd_rn(x_ma<M, R, 5>(m, TB, l2, TC, l3), __fsqrt_rn(x_dist2(l2, BCBC, BCCD, CDCD))));
-  }
-  fBC = fminf(fBC, fminf(eB, eC));
-  if (dAB >= 0.0f) {
-    const float sd = __fsqrt_rn(dAB);
-    l1 = x_root(__fadd_rn(-qAB, sd), pAB);
-    l2 = __fsub_rn(1.0f, l1);
-    if (l1 >= 0 && l1 <= 1)
-      fAB = fminf(fAB, __fadd_rn(x_ma<M, R, 14>(m, TA, l1, TB, l2),
-                                 __fsqrt_rn(x_dist3<M, R, 15>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-    l1 = x_root(__fsub_rn(-qAB, sd), pAB);
-    l2 = __fsub_rn(1.0f, l1);
-    if (l1 >= 0 && l1 <= 1)
-      fAB = fminf(fAB, __fadd_rn(x_ma<M, R, 19>(m, TA, l1, TB, l2),
-                                 __fsqrt_rn(x_dist3<M, R, 20>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-  }
-  fAB = fminf(fAB, fminf(eB, eA));
-  if (dAC >= 0.0f) {
-    const float sd = __fsqrt_rn(dAC);
-    l1 = x_root(__fadd_rn(-qAC, sd), pAC);
-    l3 = __fsub_rn(1.0f, l1);
-    if (l1 >= 0 && l1 <= 1)
-      fAC = fminf(fAC, __fadd_rn(x_ma<M, R, 28>(m, TA, l1, TC, l3), __fsqrt_rn(x_dist2(l1, ACAC, ACCD, CDCD))));
-    l1 = x_root(__fsub_rn(-qAC, sd), pAC);
-    l3 = __fsub_rn(1.0f, l1);
-    if (l1 >= 0 && l1 <= 1)
-      fAC = fminf(fAC, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 29>(m, TA, l1, TB, 0.0f)),
-                                 __fsqrt_rn(x_dist2(l1, ACAC, ACCD, CDCD))));
-  }
-  fAC = fminf(fAC, fminf(eA, eC));
-  if (delta >= 0.0f) {
-    const float sd = __fsqrt_rn(delta);
-    l1 = x_root(__fadd_rn(-q, sd), p);
-    l2 = small_quot(__fmaf_rn(s, l1, t), h);
-    l3 = __fsub_rn(__fsub_rn(1.0f, l1), l2);
-    if (l1 >= 0 && l1 <= 1 && l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)
-      TD = fminf(TD, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 42>(m, TA, l1, TB, l2)),
-                               __fsqrt_rn(x_dist3<M, R, 43>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-    l1 = x_root(__fsub_rn(-q, sd), p);
-    l2 = small_quot(__fmaf_rn(s, l1, t), h);
-    l3 = __fsub_rn(__fsub_rn(1.0f, l1), l2);
-    if (l1 >= 0 && l1 <= 1 && l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)
-      TD = fminf(TD, __fadd_rn(__fmaf_rn(TC, l3, x_ma<M, R, 47>(m, TA, l1, TB, l2)),
-                               __fsqrt_rn(x_dist3<M, R, 48>(m, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
-  }
-  return fminf(TD, fminf(fBC, fminf(fAB, fAC)));
+  const float qAC = x_ms(f.abc, __fmul_rn(__fadd_rn(ACCD, ACCD), TAC), TAC, __fmul_rn(2.0f, ACAC), ACCD);
+  const float rAC = __fmaf_rn(TAC2, CDCD, -__fmul_rn(ACCD, ACCD));
+  const float s = __fmaf_rn(TAC, ACBC, -__fmul_rn(TBC, ACAC));
+  const float t = x_ms(f.c, TAC, BCCD, TBC, ACCD);
+  const float h = -__fmaf_rn(-TBC, ACBC, __fmul_rn(TAC, BCBC));
+  const float A1 = __fmaf_rn(TAC2, ACAC, -__fmul_rn(ACAC, ACAC));
+  const float A2 = __fmaf_rn(__fmul_rn(BCBC, TAC), TAC, -__fmul_rn(ACBC, ACBC));
+  const float A3 = x_ms(f.ab, __fmul_rn(__fadd_rn(ACBC, ACBC), TAC), TAC, __fmul_rn(2.0f, ACAC), ACBC);
+  const float A4 = x_ms(f.c, __fmul_rn(__fadd_rn(BCCD, BCCD), TAC), TAC, __fmul_rn(2.0f, ACBC), ACCD);
+  o.p = __fmaf_rn(__fmul_rn(A3, s), h, __fmaf_rn(__fmul_rn(A2, s), s, __fmul_rn(__fmul_rn(A1, h), h)));
+  o.q = __fmaf_rn(__fmul_rn(A4, s), h,
+                  __fmaf_rn(__fmul_rn(qAC, h), h,
+                            __fmaf_rn(__fmul_rn(__fmul_rn(A2, 2.0f), s), t, __fmul_rn(__fmul_rn(A3, t), h))));
+  const float r = __fmaf_rn(__fmul_rn(rAC, h), h,
+                            __fmaf_rn(__fmul_rn(__fmaf_rn(TAC2, BCBC, -__fmul_rn(ACBC, ACBC)), t), t,
+                                      __fmul_rn(__fmul_rn(A4, t), h)));
+  const float delta = __fmaf_rn(o.q, o.q, -__fmul_rn(__fmul_rn(4.0f, o.p), r));
+  o.s = s;
+  o.t = t;
+  o.h = h;
+  o.sd = (delta >= 0.0f) ? __fsqrt_rn(delta) : -1.0f;
+  return o;
 }
-
-#ifndef EIK_TET_BRANCHFREE
-#define EIK_TET_BRANCHFREE 0
-#endif
-#if EIK_TET_BRANCHFREE == 1
-#define EIK_TET_UPDATE tet_update_xb
-#elif EIK_TET_BRANCHFREE == 2
-#define EIK_TET_UPDATE tet_update_xd
-#else
-#define EIK_TET_UPDATE tet_update_x
-#endif
+__device__ __forceinline__ float tet_inner_root(const TetInner& o, bool minus, ApexFuse f, float TA, float TB, float TC,
+                                                float ACAC, float ACBC, float ACCD, float BCBC, float BCCD,
+                                                float CDCD) {
+  const float l1 = x_root(__fadd_rn(-o.q, minus ? -o.sd : o.sd), o.p);
+  if (!(l1 >= 0 && l1 <= 1)) return kLarge3DDev;
+  const float l2 = small_quot(__fmaf_rn(o.s, l1, o.t), o.h);
+  const float l3 = __fsub_rn(__fsub_rn(1.0f, l1), l2);
+  if (!(l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)) return kLarge3DDev;
+  return fminf(kLarge3DDev, __fadd_rn(__fmaf_rn(TC, l3, __fmaf_rn(TA, l1, __fmul_rn(TB, l2))),
+                                      __fsqrt_rn(x_dist3(f, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
+}
+// The whole update of apex k's argument order; out of line, one body for all apex kinds,
+// which spares the instruction cache and lets a warp's lanes update different apexes.
+__device__ __noinline__ float tet_update_whole(int k, float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
+                                               float BCBC, float BCCD, float CDCD) {
+  if (TA >= kLarge3DDev && TB >= kLarge3DDev && TC >= kLarge3DDev) return kLarge3DDev;
+  const ApexFuse f = apex_fuse(k);
+  float best = fminf(tet_part_edge(false, f, TB, TC, BCBC, BCCD, CDCD), tet_part_edge(true, f, TA, TC, ACAC, ACCD, CDCD));
+  best = fminf(best, tet_part_ab(f, TA, TB, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+  const TetInner o = tet_inner_setup(f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
+  if (o.sd >= 0.0f) {
+    best = fminf(best, tet_inner_root(o, false, f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+    best = fminf(best, tet_inner_root(o, true, f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+  }
+  return best;
+}
 
 // The remaining metric edge products of a slot from its six stored ones
 // (CUDA_kernels.cu:429-437), in the order the tet updates take them.
@@ -639,80 +423,15 @@ __device__ __forceinline__ TetGram tet_gram9(float ACBC, float BCCD, float ACCD,
   return g;
 }
 
-#ifndef EIK_TET_NOINLINE
-#define EIK_TET_NOINLINE 1
-#endif
-#ifndef EIK_TET_ONEBODY
-#define EIK_TET_ONEBODY 2
-#endif
-#if EIK_TET_ONEBODY == 2
-// two out-of-line bodies: apexes A, B and C share one (their masks differ at 8
-// sites, taken at run time through selects), apex D has its own: little code for
-// the instruction cache, few selects (65^3 sweep kernel 2% faster than one body for
-// all four kinds, 4-6% faster than one body per mask; same bits)
-constexpr unsigned long long kFuseAll = kFuseApexA & kFuseApexB & kFuseApexC;
-constexpr unsigned long long kFuseRt = (kFuseApexA ^ kFuseApexB) | (kFuseApexA ^ kFuseApexC);
-__device__ __noinline__ float tet_update_rt(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                            float BCBC, float BCCD, float CDCD, unsigned long long m) {
-  return EIK_TET_UPDATE<kFuseAll, kFuseRt>(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD, m);
-}
-__device__ __noinline__ float tet_update_d(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                           float BCBC, float BCCD, float CDCD) {
-  return EIK_TET_UPDATE<kFuseApexD>(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
-}
-template <unsigned long long M>
-__device__ __forceinline__ float tet_update_call(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                                 float BCBC, float BCCD, float CDCD) {
-  if constexpr (M == kFuseApexD) return tet_update_d(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
-  else return tet_update_rt(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD, M);
-}
-#elif EIK_TET_ONEBODY
-// one out-of-line body for all four apex kinds: the sites where their masks agree
-// are fixed at compile time, the 13 others (kFuseRt) follow the kind's mask at run
-// time through selects; a third of the code for the instruction cache (65^3 sweep
-// kernel 2-4% faster than one body per mask, same bits)
-constexpr unsigned long long kFuseAll = kFuseApexA & kFuseApexB & kFuseApexC & kFuseApexD;
-constexpr unsigned long long kFuseRt =
-    (kFuseApexA ^ kFuseApexB) | (kFuseApexA ^ kFuseApexC) | (kFuseApexA ^ kFuseApexD);
-__device__ __noinline__ float tet_update_rt(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                            float BCBC, float BCCD, float CDCD, unsigned long long m) {
-  return EIK_TET_UPDATE<kFuseAll, kFuseRt>(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD, m);
-}
-template <unsigned long long M>
-__device__ __forceinline__ float tet_update_call(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                                 float BCBC, float BCCD, float CDCD) {
-  return tet_update_rt(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD, M);
-}
-#elif EIK_TET_NOINLINE
-// one out-of-line body per mask (apexes A and B share theirs): less code for the
-// instruction cache than four inlined copies (the item sweep kernel ran 6% faster on
-// the 65^3 workload, same bits)
-template <unsigned long long M>
-__device__ __noinline__ float tet_update_call(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                              float BCBC, float BCCD, float CDCD) {
-  return EIK_TET_UPDATE<M>(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
-}
-#else
-template <unsigned long long M>
-__device__ __forceinline__ float tet_update_call(float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                                 float BCBC, float BCCD, float CDCD) {
-  return EIK_TET_UPDATE<M>(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
-}
-#endif
-
-// The update of apex k (0..3 = A, B, C, D) of a slot with corner times T, as the
-// reference's FIMCuda computes it for that apex (its arguments and its roundings).
-template <int K>
-__device__ __forceinline__ float apex_update(const float T[4], const TetGram& g) {
-  if constexpr (K == 3)
-    return tet_update_call<kFuseApexD>(T[0], T[1], T[2], g.ACAC, g.ACBC, g.ACCD, g.BCBC, g.BCCD, g.CDCD);
-  if constexpr (K == 0)
-    return tet_update_call<kFuseApexA>(T[1], T[3], T[2], g.BCBC, -g.BCCD, -g.ACBC, g.CDCD, g.ACCD, g.ACAC);
-  if constexpr (K == 1)
-    return tet_update_call<kFuseApexB>(T[0], T[3], T[2], g.ACAC, -g.ACCD, -g.ACBC, g.CDCD, g.BCCD, g.BCBC);
-  if constexpr (K == 2)
-    return tet_update_call<kFuseApexC>(T[0], T[1], T[3], g.ADAD, g.ADBD, -g.ADCD, g.BDBD, -g.CDBD, g.CDCD);
-  return kLarge3DDev;
+// An apex update's arguments: the times of its face's corners and the metric products
+// as the reference passes them for apex k (0..3 = A, B, C, D).  k may differ between the
+// lanes of a warp: every argument is picked by selects.
+__device__ __forceinline__ float apex_update(int k, const float T[4], const TetGram& g) {
+  const bool a = k == 0, c = k == 2, ab = k < 2;
+  return tet_update_whole(k, a ? T[1] : T[0], ab ? T[3] : T[1], c ? T[3] : T[2], a ? g.BCBC : c ? g.ADAD : g.ACAC,
+                          a ? -g.BCCD : c ? g.ADBD : ab ? -g.ACCD : g.ACBC, ab ? -g.ACBC : c ? -g.ADCD : g.ACCD,
+                          ab ? g.CDCD : c ? g.BDBD : g.BCBC, a ? g.ACCD : c ? -g.CDBD : g.BCCD,
+                          a ? g.ACAC : ab ? g.BCBC : g.CDCD);
 }
 
 // The operations of the wide (precision mode) update, named so the update reads

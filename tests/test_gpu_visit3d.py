@@ -1,0 +1,70 @@
+"""The 3D item visit (copies put off, one update body for all apexes) against the
+slot-per-thread kernels, which run precision mode with no tet flagged: results, iteration
+and visit counts are equal, bit for bit, over block shapes around a CTA's and a warp's
+size, scalar and anisotropic metrics, slivers, caps and several seeds."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(mg, mesh, n):
+    xyz, tets = mg.kuhn_cube(n, 0.0 if mesh == "flat" else 0.2, seed=n)
+    if mesh == "layers":  # a thin layer: slivers
+        xyz = xyz.copy()
+        z = xyz[:, 2]
+        xyz[:, 2] = np.where(z > 0.5, z - 0.97 / (n - 1) * np.minimum(1.0, (z - 0.5) * (n - 1)), z)
+    return xyz, tets
+
+
+def _solve(eik, xyz, tets, metric, seeds, vpb, cap, slots, **opts):
+    e = eik.Eikonal(False)
+    e.set_mesh(xyz, tets)
+    e.maxVertsPerBlock_ = vpb
+    e.maxIterations_ = cap
+    for k, v in opts.items():
+        setattr(e, k, v)
+    if slots:
+        e.precisionMode_ = 1
+        e.precisionKappa_ = 1e30
+    if metric is not None:
+        e.initSpeedMtxMultipliers(metric)
+    e.setSeeds(seeds)
+    e.solveEikonal()
+    first = e.getFinalResult().view(np.uint32).copy()
+    e.solveEikonal()
+    assert np.array_equal(first, e.getFinalResult().view(np.uint32))
+    s = e.stats()
+    assert s["flagged_tets"] == 0
+    return [first, np.array([s[k] for k in ("iterations", "vertex_updates", "fim_visits", "check_visits")])] + [
+        e.getResultAtIteration(i).view(np.uint32) for i in range(e.numIterations())]
+
+
+@pytest.mark.parametrize("mesh,n,vpb,metric,seeds,cap", [
+    ("cube", 3, 64, 1, [0], 100),
+    ("cube", 5, 2, 1, [0, 100], 200),
+    ("cube", 9, 8, 1, [0], 200),
+    ("cube", 13, 33, 6, [5, 1000], 200),
+    ("cube", 17, 64, 1, [0, 2000, 4912], 100),
+    ("cube", 17, 64, 0, [2456], 100),
+    ("flat", 17, 64, 0, [2456], 100),
+    ("cube", 21, 100, 1, [7], 200),
+    ("layers", 17, 64, 6, [0, 4000], 300),
+    ("layers", 15, 48, 1, [1687], 300),
+    ("cube", 25, 64, 6, [0, 7812, 15000], 1),
+    ("cube", 25, 64, 1, [0, 7812, 15000], 2),
+    ("cube", 25, 64, 1, [0, 7812, 15000], 7),
+])
+def test_item_visits_equal_slot_kernels(eik, mg, mesh, n, vpb, metric, seeds, cap):
+    xyz, tets = _mesh(mg, mesh, n)
+    m = None
+    if metric == 1:
+        m = (1.0 / mg.log_uniform_speeds(tets.shape[0], seed=n).astype(np.float64) ** 2).astype(np.float32)
+    elif metric == 6:
+        m = mg.anisotropic_metrics(tets.shape[0], seed=n)
+    got = _solve(eik, xyz, tets, m, seeds, vpb, cap, False)
+    want = _solve(eik, xyz, tets, m, seeds, vpb, cap, True)
+    one_by_one = _solve(eik, xyz, tets, m, seeds, vpb, cap, False, directLaunch_=1)
+    for other in (want, one_by_one):
+        assert len(got) == len(other)
+        assert all(np.array_equal(a, b) for a, b in zip(got, other))
