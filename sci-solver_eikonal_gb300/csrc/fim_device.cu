@@ -1302,7 +1302,7 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
     const int ist = done1 >= 0 ? done1 : a.inst_done[a.blk_inst[b]];
     bool sweep = ist == 0;
     if (ist != 1 && (sweep || chk)) {
-      if (!load_visit3d(a, bd, s, &bar, parity, chk ? a.chk_memo : a.fim_memo)) {
+      if (!load_visit3d(a, bd, s, &bar, parity, a.Ta, chk ? a.chk_memo : a.fim_memo)) {
         if (tid == 0) atomicOr(&a.ctl->error, kErrWait);
         (void)mbar_wait(&bar, parity ^ 1u);
         sweep = false;
@@ -1310,7 +1310,7 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
         __syncthreads();
         const int nown = bd.nowned;
         if (chk) {
-          const bool moved = check_visit3d(a, bd, s, s_n, &s_moved);
+          const bool moved = check_visit3d(a, bd, s, s_n, &s_moved, [] {});
           if (tid == 0) {  // the previous iteration's check (run_check_neghbor)
             atomicAdd(&ctl->chk_visits, 1ull);
             atomicAdd(&ctl->updates, (unsigned long long)nown);
@@ -1323,7 +1323,7 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
           sweep = sweep && moved;
         }
         if (sweep) {
-          sweep_visit3d(a, bd, s, s_n, chk);
+          sweep_visit3d(a, bd, s, s_n, chk, true, [] {});
           int myconv = 1;
           for (int k = tid; k < nown; k += NT) {
             const float ov = __int_as_float(s.v1[k]), nv = __int_as_float(s.v2[k]);
@@ -2070,6 +2070,8 @@ __global__ void k_close3d(DevArgs a, int copy) {
   finish_iteration_cta(a, false);
 }
 
+#include "loop3d.cuh"
+
 // start of a solve: set the while-condition from the initial active list
 // initial travel times: LARGENUM everywhere (prev too unless the caller's initial
 // values were copied in) ...
@@ -2555,6 +2557,8 @@ struct DeviceSolve::Impl {
   int* inst_fail = nullptr;
   int* inst_maxit = nullptr;
   int* inst_unreached = nullptr;
+  int* inst_bbeg = nullptr;    // 2D: first block of every instance (ninst + 1)
+  int* loop3_lists = nullptr;  // 3D loop kernel: two lists of converged blocks, memo flags
   unsigned char* stage = nullptr;  // loop kernels: control block and the solve's inputs
   size_t stage_cap = 0;
   std::vector<unsigned char> h_stage;
@@ -2642,7 +2646,7 @@ struct DeviceSolve::Impl {
     void* ps[] = {blocks, coef, lv, halo, nbr_off, nbr, vblock, perm, Ta, Tb, Tinit, prev, conv,
                   stampA, stampC, visited, list0, list1, list_new, ctl, hist, ktime, out_tmp,
                   blk_inst, inst_done, inst_iters, inst_nnext, inst_fail, inst_maxit, seed_ids,
-                  cand, inst_swept, inst_ncand, inst_unreached, stage, slot_f64, coef64, res_cand, inst_vbeg, chunks, chk_memo, hsb, hs64, hsu64};
+                  cand, inst_swept, inst_ncand, inst_unreached, inst_bbeg, loop3_lists, stage, slot_f64, coef64, res_cand, inst_vbeg, chunks, chk_memo, hsb, hs64, hsu64};
     for (void* p : ps)
       if (p) cudaFree(p);
     hsb = nullptr;
@@ -2666,6 +2670,8 @@ struct DeviceSolve::Impl {
     blk_inst = nullptr; inst_done = nullptr; inst_iters = nullptr; inst_nnext = nullptr; inst_fail = nullptr;
     inst_maxit = nullptr;
     inst_unreached = nullptr;
+    inst_bbeg = nullptr;
+    loop3_lists = nullptr;
     stage = nullptr;
     stage_cap = 0;
     cand = nullptr; inst_swept = nullptr; inst_ncand = nullptr;
@@ -2677,6 +2683,9 @@ struct DeviceSolve::Impl {
   void fill_args(DevArgs& a, const Layout& L, int sweeps, int hcap, bool serve, bool tele) const;
   std::string build_graph(const Layout& L, int sweeps, int threads, int hcap, bool serve);
   std::string choose_loop2d(const Layout& L);
+  std::string stage_inputs(size_t o_words, const std::vector<int>& cap, int max_iters, int** words);
+  std::string run_loop3d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap,
+                         int threads);
   std::string run_loop2d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap);
   void drop_graph() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -2776,7 +2785,72 @@ std::string DeviceSolve::Impl::run_loop2d(const Layout& L, const SolveOptions& o
   const size_t nseed = P.h_seed_ids.size(), nact = P.h_act.size(), ni = (size_t)P.ninst;
   const size_t o_flags = (sizeof(Ctl) + 127) & ~(size_t)127, o_sync = o_flags + sizeof(GridFlag) * kGridFlags;
   const size_t o_words = o_sync + sizeof(InstSync) * ni;
-  const size_t bytes = o_words + sizeof(int) * (3 * ni + 1 + nseed + nact);
+  int* w = nullptr;
+  std::string e = P.stage_inputs(o_words, cap, max_iters, &w);
+  if (!e.empty()) return e;
+  a.ctl = P.last_ctl;
+  Start2 s2{w, w + ni, w + 2 * ni, w + 2 * ni + nseed, (int)nseed, (int)nact, P.inst_bbeg,
+            reinterpret_cast<InstSync*>(P.stage + o_sync), reinterpret_cast<GridFlag*>(P.stage + o_flags),
+            P.h_prev.empty() ? 0 : 1, a.ktime ? 1 : 0};
+  if (!P.h_prev.empty())
+    CK(cudaMemcpyAsync(P.prev, P.h_prev.data(), sizeof(float) * L.nv, cudaMemcpyHostToDevice, st));
+  if (!P.loop_func && !(e = P.choose_loop2d(L)).empty()) return e;
+  CK(cudaEventRecord(P.ev0, st));
+  void* args[] = {&a, &s2};
+  CK(cudaLaunchCooperativeKernel(P.loop_func, dim3(P.loop_grid), dim3(P.loop_threads), args, P.loop_smem, st));
+  return "";
+}
+
+// One 3D solve or batch in k_loop3d, enqueued on the solver's stream.
+std::string DeviceSolve::Impl::run_loop3d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap,
+                                          int max_iters, int hcap, int threads) {
+  Impl& P = *this;
+  cudaStream_t st = (cudaStream_t)opt_stream;
+  std::string e;
+  if (!P.chk_memo) {
+    if (!(e = dev_alloc(P.chk_memo, 2 * (P.coef_n / 6))).empty()) return e;
+    P.drop_graph();
+  }
+  if (!P.loop3_lists && !(e = dev_alloc(P.loop3_lists, 3 * (size_t)L.nb)).empty()) return e;
+  DevArgs a;
+  P.fill_args(a, L, 2, hcap, false, opt.telemetry);
+  a.use_cond = 0;
+  a.fused = 1;
+  a.fim_memo = P.chk_memo + P.coef_n / 6;
+  const size_t nseed = P.h_seed_ids.size(), nact = P.h_act.size(), ni = (size_t)P.ninst;
+  const size_t o_flags = (sizeof(Ctl) + 127) & ~(size_t)127, o_turn = o_flags + sizeof(GridFlag) * kGridFlags;
+  const size_t o_words = o_turn + 3 * sizeof(Turn3);
+  int* w = nullptr;
+  if (!(e = P.stage_inputs(o_words, cap, max_iters, &w)).empty()) return e;
+  a.ctl = P.last_ctl;
+  Start3 s3{w, w + ni, w + 2 * ni, w + 2 * ni + nseed, (int)nseed, (int)nact,
+            reinterpret_cast<Turn3*>(P.stage + o_turn), reinterpret_cast<GridFlag*>(P.stage + o_flags),
+            P.loop3_lists, P.loop3_lists + 2 * (size_t)L.nb, {P.stampC, P.list_new}};
+  if (!P.loop_func || P.loop_threads != threads) {
+    int dev = 0, nsm = 0, occ = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    P.loop_smem = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned);
+    CK(raise_smem_limit((const void*)k_loop3d, P.loop_smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_loop3d, threads, P.loop_smem));
+    if (occ < 1) return "loop kernel cannot be resident (shared memory / registers)";
+    P.loop_func = (const void*)k_loop3d;
+    P.loop_threads = threads;
+    P.loop_grid = std::max(1, std::min(occ * nsm, L.nb));
+  }
+  CK(cudaEventRecord(P.ev0, st));
+  void* args[] = {&a, &s3};
+  CK(cudaLaunchCooperativeKernel(P.loop_func, dim3(P.loop_grid), dim3(threads), args, P.loop_smem, st));
+  return "";
+}
+
+// Copies a loop kernel's inputs to the device in one piece: the control block, zeros up
+// to byte o_words, then per instance its done flag and its cap, the seeds and the
+// starting blocks.  *words receives the device address of the flags.
+std::string DeviceSolve::Impl::stage_inputs(size_t o_words, const std::vector<int>& cap, int max_iters, int** words) {
+  Impl& P = *this;
+  const size_t nseed = P.h_seed_ids.size(), nact = P.h_act.size(), ni = (size_t)P.ninst;
+  const size_t bytes = o_words + sizeof(int) * (2 * ni + nseed + nact);
   if (bytes > P.stage_cap) {
     std::string e = dev_alloc(P.stage, bytes + 1024);
     if (!e.empty()) return e;
@@ -2790,24 +2864,11 @@ std::string DeviceSolve::Impl::run_loop2d(const Layout& L, const SolveOptions& o
   int* w = reinterpret_cast<int*>(P.h_stage.data() + o_words);
   for (size_t i = 0; i < ni; ++i) w[i] = (cap[i] <= 0) ? 1 : P.h_done[i];
   std::copy(cap.begin(), cap.end(), w + ni);
-  if (L.ninst > 1) std::copy(L.inst_bbeg.begin(), L.inst_bbeg.end(), w + 2 * ni);
-  else w[2 * ni + 1] = L.nb;
-  std::copy(P.h_seed_ids.begin(), P.h_seed_ids.end(), w + 3 * ni + 1);
-  std::copy(P.h_act.begin(), P.h_act.end(), w + 3 * ni + 1 + nseed);
-  CK(cudaMemcpyAsync(P.stage, P.h_stage.data(), bytes, cudaMemcpyHostToDevice, st));
-  a.ctl = P.last_ctl = reinterpret_cast<Ctl*>(P.stage);
-  const int* dw = reinterpret_cast<const int*>(P.stage + o_words);
-  Start2 s2{dw, dw + ni, dw + 3 * ni + 1, dw + 3 * ni + 1 + nseed, (int)nseed, (int)nact, dw + 2 * ni,
-            reinterpret_cast<InstSync*>(P.stage + o_sync), reinterpret_cast<GridFlag*>(P.stage + o_flags), P.h_prev.empty() ? 0 : 1, a.ktime ? 1 : 0};
-  if (!P.h_prev.empty())
-    CK(cudaMemcpyAsync(P.prev, P.h_prev.data(), sizeof(float) * L.nv, cudaMemcpyHostToDevice, st));
-  if (!P.loop_func) {
-    std::string e = P.choose_loop2d(L);
-    if (!e.empty()) return e;
-  }
-  CK(cudaEventRecord(P.ev0, st));
-  void* args[] = {&a, &s2};
-  CK(cudaLaunchCooperativeKernel(P.loop_func, dim3(P.loop_grid), dim3(P.loop_threads), args, P.loop_smem, st));
+  std::copy(P.h_seed_ids.begin(), P.h_seed_ids.end(), w + 2 * ni);
+  std::copy(P.h_act.begin(), P.h_act.end(), w + 2 * ni + nseed);
+  CK(cudaMemcpyAsync(P.stage, P.h_stage.data(), bytes, cudaMemcpyHostToDevice, (cudaStream_t)opt_stream));
+  P.last_ctl = reinterpret_cast<Ctl*>(P.stage);
+  *words = reinterpret_cast<int*>(P.stage + o_words);
   return "";
 }
 
@@ -3261,6 +3322,7 @@ std::string DeviceSolve::finish_upload(const Layout& L, bool layout_on_device) {
     if (!(e = dev_alloc(*t, (size_t)P.ninst)).empty()) return e;
   if (!(e = dev_alloc(P.cand, 2 * (size_t)L.nb)).empty()) return e;
   if (!(e = dev_alloc(P.inst_vbeg, (size_t)P.ninst + 1)).empty()) return e;
+  if (!(e = dev_alloc(P.inst_bbeg, (size_t)P.ninst + 1)).empty()) return e;
   cudaStream_t st = (cudaStream_t)stream_;
   std::vector<int>& vb = P.h_vblock;
   vb.assign(L.nv, 0);
@@ -3292,6 +3354,9 @@ std::string DeviceSolve::finish_upload(const Layout& L, bool layout_on_device) {
   std::vector<int> bi(L.blk_inst);
   if ((int)bi.size() != L.nb) bi.assign(L.nb, 0);
   CK(cudaMemcpyAsync(P.blk_inst, bi.data(), sizeof(int) * L.nb, cudaMemcpyHostToDevice, st));
+  std::vector<int> bb0(L.inst_bbeg);
+  if ((int)bb0.size() != P.ninst + 1) bb0 = {0, L.nb};
+  CK(cudaMemcpyAsync(P.inst_bbeg, bb0.data(), sizeof(int) * bb0.size(), cudaMemcpyHostToDevice, st));
   std::vector<int> vb0(L.inst_vbeg);
   if ((int)vb0.size() != P.ninst + 1) vb0 = {0, L.nv};
   CK(cudaMemcpyAsync(P.inst_vbeg, vb0.data(), sizeof(int) * vb0.size(), cudaMemcpyHostToDevice, st));
@@ -3413,6 +3478,8 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   }
   // 2D solves of the reference's seven sweeps run in one resident kernel (k_loop2d)
   const bool loop2d = L.dim == 2 && sweeps == 7 && !opt.direct_launch && P.max_slots_pad <= 1024;
+  // 3D ones of its two sweeps in another (k_loop3d)
+  const bool loop3d = L.dim == 3 && items && sweeps == 2 && !opt.direct_launch;
   // per-instance iteration caps (one cap for all when not given)
   std::vector<int> cap(P.ninst, opt.max_iterations);
   if ((int)opt.inst_max_iterations.size() == P.ninst) cap = opt.inst_max_iterations;
@@ -3442,6 +3509,10 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   bool tele = false;  // whether this solve recorded its launches
   if (loop2d) {
     std::string e = P.run_loop2d(L, opt, cap, max_iters, hcap);
+    if (!e.empty()) return e;
+    tele = opt.telemetry;
+  } else if (loop3d) {
+    std::string e = P.run_loop3d(L, opt, cap, max_iters, hcap, threads);
     if (!e.empty()) return e;
     tele = opt.telemetry;
   } else {

@@ -53,6 +53,7 @@ __device__ __forceinline__ bool grid_wait(GridBar* g, const unsigned* word, unsi
   unsigned long long t0 = 0;
   for (unsigned i = 0;; ++i) {
     if ((int)(ld_acquire(word) - want) >= 0) return true;
+    if (i > 4) __nanosleep(32);
     if ((i & 255u) == 255u) {
       if (ld_acquire(&g->fail)) return false;
       const unsigned long long t = global_ns();

@@ -72,7 +72,8 @@ __device__ __forceinline__ SmemV carve_visit3d(unsigned char* sm, const DevArgs&
 // Loads block bd: the bulk copies of its coefficients, corner ids, bounds and `memo`
 // entries (into h0), its owned and halo times from Tsrc.  Returns false on a timeout.
 __device__ __forceinline__ bool load_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s,
-                                             unsigned long long* bar, unsigned& parity, const uint4* memo) {
+                                             unsigned long long* bar, unsigned& parity, const float* Tsrc,
+                                             const uint4* memo) {
   const int tid = threadIdx.x, NT = blockDim.x;
   if (tid == 0) {
     fence_proxy_async();
@@ -86,11 +87,11 @@ __device__ __forceinline__ bool load_visit3d(const DevArgs& a, const BlockDesc& 
     }
   }
   for (int k = tid; k < bd.nowned; k += NT) {
-    const float v = __ldcg(a.Ta + bd.vbase + k);
+    const float v = __ldcg(Tsrc + bd.vbase + k);
     s.vt[k] = v;
     s.v1[k] = __float_as_int(v);  // times are never negative: their bits order as integers do
   }
-  for (int k = tid; k < bd.nhalo; k += NT) s.vt[bd.nowned + k] = __ldcg(a.Ta + a.halo[bd.halo_begin + k]);
+  for (int k = tid; k < bd.nhalo; k += NT) s.vt[bd.nowned + k] = __ldcg(Tsrc + a.halo[bd.halo_begin + k]);
   const bool ok = mbar_wait(bar, parity);
   parity ^= 1u;
   return ok;
@@ -178,8 +179,10 @@ __device__ __forceinline__ void run_items(const BlockDesc& bd, const SmemV& s, i
 
 // One check of a loaded block (its check memos in h0): whether it moves.  s_n: two
 // counters, zero on entry and on return.  All threads; ends behind a CTA barrier.
+// `aside` runs in the CTA's last warp while the others update: the items seldom reach it.
+template <class Aside>
 __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, int* s_n,
-                                              volatile int* s_moved) {
+                                              volatile int* s_moved, Aside aside) {
   const int tid = threadIdx.x, NT = blockDim.x, ns = bd.nslots, nown = bd.nowned;
   if (tid == 0) *s_moved = 0;
   for (int j0 = 0; j0 < ns; j0 += NT) {
@@ -205,6 +208,7 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
     append_items(s.items, s_n, need, j);
   }
   __syncthreads();
+  if (tid >= NT - 32) aside();
   run_items<0>(bd, s, s_n[0], s_moved);
   __syncthreads();
   const bool moved = *s_moved != 0;
@@ -222,10 +226,11 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
 }
 
 // The two sweeps of a loaded block (its sweep memos in h0, or behind a check read from
-// memory): the final owned times in v2, those after the first sweep in v1.  s_n as above.
+// memory, where `memo` says they are of this solve): the final owned times in v2, those after the first sweep in v1.  s_n as above.
 // Ends behind a CTA barrier.
+template <class Aside>
 __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, int* s_n,
-                                              bool checked) {
+                                              bool checked, bool memo, Aside aside) {
   const int tid = threadIdx.x, NT = blockDim.x, ns = bd.nslots, nown = bd.nowned;
   // ---- first sweep: owned apexes; bounds of the copies ----
   for (int j0 = 0; j0 < ns; j0 += NT) {
@@ -241,7 +246,7 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
       slot_bounds(s.hs[j], hs);
       unsigned same = 0, live = 0, own = 0;
       if (!checked) same = same_bits(T, reinterpret_cast<const uint4*>(s.h0)[j]);
-      else if (s.fl[j]) same = same_bits(T, a.fim_memo[bd.slot_begin + j]);
+      else if (s.fl[j] && memo) same = same_bits(T, __ldcg(a.fim_memo + bd.slot_begin + j));
       float lo[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -313,6 +318,7 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
     }
   }
   __syncthreads();
+  if (tid >= NT - 32) aside();
   run_items<1>(bd, s, s_n[0], nullptr);
   __syncthreads();
   const int nd = s_n[1];

@@ -68,3 +68,64 @@ def test_item_visits_equal_slot_kernels(eik, mg, mesh, n, vpb, metric, seeds, ca
     for other in (want, one_by_one):
         assert len(got) == len(other)
         assert all(np.array_equal(a, b) for a, b in zip(got, other))
+
+
+def test_batch_with_caps_equals_single_solves(eik, mg):
+    """Instances that stop at their caps keep their times while the others run on."""
+    hs = []
+    for i, (n, cap) in enumerate([(9, 1), (13, 4), (17, 1000), (21, 6), (7, 0), (15, 1000), (17, 11)]):
+        xyz, tets = mg.kuhn_cube(n, 0.2, seed=n)
+        e = eik.Eikonal(False)
+        e.set_mesh(xyz, tets)
+        e.maxIterations_ = cap
+        e.keepHistory_ = 0
+        e.initSpeedMtxMultipliers(mg.log_uniform_speeds(tets.shape[0], seed=i))
+        e.setSeeds([i, xyz.shape[0] // 2])
+        hs.append(e)
+    b = eik.EikonalBatch(hs)
+    for _ in range(2):
+        b.solveEikonal()
+        res = [r.copy() for r in b.getFinalResults()]
+        total = b.stats()
+        visits = np.zeros(4, np.int64)
+        for i, h in enumerate(hs):
+            h.directLaunch_ = 1
+            h.solveEikonal()
+            h.directLaunch_ = 0
+            s = h.stats()
+            visits += [s["vertex_updates"], s["fim_visits"], s["check_visits"], s["slot_visits"]]
+            assert np.array_equal(res[i].view(np.uint32), h.getFinalResult().view(np.uint32)), i
+            assert b.numIterations(i) == h.numIterations()
+        assert visits.tolist() == [total[k] for k in ("vertex_updates", "fim_visits", "check_visits", "slot_visits")]
+
+
+def test_concurrent_solves_of_several_threads(eik, mg):
+    """Loop kernels that each fill the GPU, launched from four threads at once."""
+    import threading
+
+    hs, want, failures = [], [], []
+    for i in range(4):
+        xyz, tets = mg.kuhn_cube(27 + i, 0.2, seed=i)
+        e = eik.Eikonal(False)
+        e.set_mesh(xyz, tets)
+        e.keepHistory_ = 0
+        e.setSeeds([i])
+        e.solveEikonal()
+        hs.append(e)
+        want.append(e.getFinalResult().view(np.uint32).copy())
+
+    def work(h, w):
+        try:
+            for _ in range(5):
+                h.solveEikonal()
+                if not np.array_equal(h.getFinalResult().view(np.uint32), w):
+                    failures.append("bits")
+        except Exception as ex:  # reported below
+            failures.append(repr(ex))
+
+    ts = [threading.Thread(target=work, args=x) for x in zip(hs, want)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not failures
