@@ -236,6 +236,12 @@ constexpr int kKStride = 16;    // words of per-iteration telemetry (DevArgs::kt
 #ifndef EIK_ITEM_MAXNREG
 #define EIK_ITEM_MAXNREG 56
 #endif
+#ifndef EIK_PREC_THREADS
+#define EIK_PREC_THREADS 384
+#endif
+#ifndef EIK_PREC_MAXNREG
+#define EIK_PREC_MAXNREG 80
+#endif
 // sweep visits: the block's sweep memos arrive with its bulk copies (1) or are read
 // from memory while the first sweep's updates are listed (0)
 #ifndef EIK_STAGE_SWEEP_MEMO
@@ -1267,14 +1273,15 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a, int role) {
 // by the previous iteration's commit; a candidate that moves is appended to this
 // iteration's active list and swept in the same visit.
 // ===========================================================================
-__global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
+template <bool kPrec>
+__global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
   pdl_begin();
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int s_item;
-  __shared__ int s_n[2];
+  __shared__ int s_n[6];
   __shared__ volatile int s_moved;
-  const SmemV s = carve_visit3d(sm, a);
+  const SmemV s = carve_visit3d<kPrec>(sm, a);
   const int tid = threadIdx.x, NT = blockDim.x;
   Ctl* ctl = a.ctl;
   const int iter = ctl->iter;
@@ -1283,9 +1290,10 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
   const int* cand = a.cand + (size_t)((iter + 1) & 1) * a.nb;
   const int count = nact + ctl->ncand[(iter + 1) & 1];
   int* list = act_list(a, iter);
+  const PrecMode pm = kPrec ? PrecMode{ctl->f64_all, ctl->polish} : PrecMode{0, 0};
   stamp_start(a, iter, 0);
   if (tid == 0) mbar_init(&bar, 1);
-  if (tid < 2) s_n[tid] = 0;
+  if (tid < 6) s_n[tid] = 0;
   __syncthreads();
   unsigned parity = 0;
   // the first block of a CTA is its own index; later ones come from the counter
@@ -1309,8 +1317,12 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
       } else {
         __syncthreads();
         const int nown = bd.nowned;
+        if constexpr (kPrec) {
+          load_prec3d(a, bd, s, pm);
+          __syncthreads();
+        }
         if (chk) {
-          const bool moved = check_visit3d(a, bd, s, s_n, &s_moved, [] {});
+          const bool moved = check_visit3d<kPrec>(a, bd, s, s_n, &s_moved, [] {}, pm);
           if (tid == 0) {  // the previous iteration's check (run_check_neghbor)
             atomicAdd(&ctl->chk_visits, 1ull);
             atomicAdd(&ctl->updates, (unsigned long long)nown);
@@ -1323,13 +1335,13 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
           sweep = sweep && moved;
         }
         if (sweep) {
-          sweep_visit3d(a, bd, s, s_n, chk, true, [] {});
+          sweep_visit3d<kPrec>(a, bd, s, s_n, chk, true, [] {}, pm);
           int myconv = 1;
           for (int k = tid; k < nown; k += NT) {
             const float ov = __int_as_float(s.v1[k]), nv = __int_as_float(s.v2[k]);
             float res = ov - nv;
             if (res < 0.0f) res = -res;
-            myconv &= (res <= kEps3DLe) ? 1 : 0;
+            myconv &= (res <= settle_eps(ov, pm.polish)) ? 1 : 0;
             a.Tb[bd.vbase + k] = nv;
           }
           const int allc = __syncthreads_and(myconv);
@@ -2830,7 +2842,7 @@ std::string DeviceSolve::Impl::run_loop3d(const Layout& L, const SolveOptions& o
     int dev = 0, nsm = 0, occ = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    P.loop_smem = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned);
+    P.loop_smem = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, false);
     CK(raise_smem_limit((const void*)k_loop3d, P.loop_smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_loop3d, threads, P.loop_smem));
     if (occ < 1) return "loop kernel cannot be resident (shared memory / registers)";
@@ -2886,6 +2898,7 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     // 2D blocks of up to 1024 slots use the thread-per-slot kernel (bitwise equal
     // to the reference); larger 2D blocks fall back to the slot-loop kernel
+    bool items2 = false;  // the visits of the reference's two sweeps (k_items3d)
     const bool slot2d = (L.dim == 2) && P.max_slots_pad <= 1024;
     int vthreads = threads;
     size_t vsmem = P.smem, vsmem_chk = P.smem;
@@ -2930,14 +2943,15 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
         else if (!P.prec) kv_fim = (void*)k_visit3d<false>;
 #endif
         // the reference's two sweeps have a kernel of their own
-        const size_t sv = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned);
-        if (!P.prec && sweeps == 2 && P.chk_memo && sv + 64 <= (size_t)maxsm) {
-          kv_fim = (void*)k_items3d;
+        const size_t sv = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, P.prec);
+        if (sweeps == 2 && P.chk_memo && sv + 64 <= (size_t)maxsm) {
+          items2 = true;
+          kv_fim = P.prec ? (void*)k_items3d<true> : (void*)k_items3d<false>;
           vsmem = sv;
           a.chk_memo = P.chk_memo;
         }
 #if EIK_SWEEP_MEMO
-        if ((kv_fim == (void*)k_sweep3d || kv_fim == (void*)k_items3d) && P.chk_memo)
+        if ((kv_fim == (void*)k_sweep3d || items2) && P.chk_memo)
           a.fim_memo = P.chk_memo + P.coef_n / 6;
 #endif
 #if EIK_CHECK_ITEMS
@@ -2947,7 +2961,7 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
         (void)si;
         (void)sc;
       }
-      a.fused = (kv_fim == (void*)k_items3d || (EIK_FUSED_CHECK && kv_fim == (void*)k_sweep3d && kv_chk == (void*)k_check3d)) ? 1 : 0;
+      a.fused = (items2 || (EIK_FUSED_CHECK && kv_fim == (void*)k_sweep3d && kv_chk == (void*)k_check3d)) ? 1 : 0;
     } else if (slot2d) {
       vthreads = std::max(32, (P.max_slots_pad + 31) & ~31);
       vsmem = vsmem_chk = smem_bytes_slot2d(P.max_slots_pad, P.max_local, P.max_owned);
@@ -3459,10 +3473,19 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
     CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     items = smem_bytes_items(P.max_slots_pad, P.max_local, P.max_owned) + 64 <= (size_t)maxsm;
   }
+  bool items64 = false;  // precision mode's item visits
+  if (L.dim == 3 && P.prec && sweeps == 2) {
+    int maxsm = 0, dev = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    items64 = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, true) + 64 <= (size_t)maxsm;
+  }
   if (!given && items) {
     // item kernels: 384-thread CTAs, three per SM where their shared memory allows
     // (65^3 workload: solve 7.85 ms against 7.93 at 512 and 8.4 at one thread per slot)
     threads = kItemThreads;
+  } else if (!given && items64) {
+    threads = EIK_PREC_THREADS;
   } else if (!given && L.dim == 3) {
     const int full = threads, half = auto_visit_threads(P.max_slots_pad);
     if (half < full) {

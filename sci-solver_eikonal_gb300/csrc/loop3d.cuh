@@ -175,7 +175,7 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_loop3d(const __grid_constant__ D
   __shared__ int s_n[2];
   __shared__ volatile int s_moved;
   __shared__ unsigned s_cnt[12];  // visits, slots, halo, owned of sweeps, checks and sweeps behind a check
-  const SmemV s = carve_visit3d(sm, a);
+  const SmemV s = carve_visit3d<false>(sm, a);
   GridBar* const g = &a.ctl->bar;
   const int tid = threadIdx.x, lane = tid & 31, NT = blockDim.x;
   const int G = gridDim.x, gtid = blockIdx.x * NT + tid, gn = G * NT;

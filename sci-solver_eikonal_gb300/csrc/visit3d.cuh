@@ -37,24 +37,32 @@ struct SmemV {
   unsigned short* items;  // 4 slot + apex, at most 4 per slot
   unsigned short* defer;  // slots whose copies the second sweep needs
   unsigned char* fl;      // per slot: copies of unknown value (bits 0-3), settled by the check memo (bit 7)
+  int* sf;                // precision mode: per slot the FP64 products of its tet, or -1
+  unsigned short* items64;  // ... slots of the listed FP64 updates, one list of `pitch` per apex
+  int pitch;
 };
-__host__ __device__ inline size_t visit3d_offsets(int np, int max_local, int max_owned, size_t off[10]) {
+// Precision mode (kPrec): the updates of flagged tets, and in the polish of all, run in
+// FP64.  They are listed apart, one list per apex kind, so that every FP64 instruction of
+// a warp works for all of its lanes: the FP64 unit takes 16 cycles for a warp whatever
+// the number of lanes in use, and it is what bounds the mode.
+__host__ __device__ inline size_t visit3d_offsets(int np, int max_local, int max_owned, bool prec, size_t off[12]) {
   size_t o = 0;
-  const size_t n = (size_t)np, bytes[10] = {24 * n, 8 * n, 8 * n, 16 * n, 4 * (size_t)max_local, 4 * (size_t)max_owned,
-                                            4 * (size_t)max_owned, 8 * n, 2 * n, n};
-  for (int i = 0; i < 10; ++i) {
+  const size_t n = (size_t)np, bytes[12] = {24 * n, 8 * n, 8 * n, 16 * n, 4 * (size_t)max_local, 4 * (size_t)max_owned,
+                                            4 * (size_t)max_owned, 8 * n, 2 * n, n, prec ? 4 * n : 0, prec ? 8 * n : 0};
+  for (int i = 0; i < 12; ++i) {
     off[i] = o;
     o += (bytes[i] + 15) & ~(size_t)15;
   }
   return o;
 }
-__host__ __device__ inline size_t smem_bytes_visit3d(int np, int max_local, int max_owned) {
-  size_t off[10];
-  return visit3d_offsets(np, max_local, max_owned, off);
+__host__ __device__ inline size_t smem_bytes_visit3d(int np, int max_local, int max_owned, bool prec) {
+  size_t off[12];
+  return visit3d_offsets(np, max_local, max_owned, prec, off);
 }
+template <bool kPrec>
 __device__ __forceinline__ SmemV carve_visit3d(unsigned char* sm, const DevArgs& a) {
-  size_t off[10];
-  visit3d_offsets(a.max_slots_pad, a.max_local, a.max_owned, off);
+  size_t off[12];
+  visit3d_offsets(a.max_slots_pad, a.max_local, a.max_owned, kPrec, off);
   SmemV s;
   s.coef = reinterpret_cast<float*>(sm + off[0]);
   s.lv = reinterpret_cast<uint2*>(sm + off[1]);
@@ -66,7 +74,44 @@ __device__ __forceinline__ SmemV carve_visit3d(unsigned char* sm, const DevArgs&
   s.items = reinterpret_cast<unsigned short*>(sm + off[7]);
   s.defer = reinterpret_cast<unsigned short*>(sm + off[8]);
   s.fl = sm + off[9];
+  s.sf = reinterpret_cast<int*>(sm + off[10]);
+  s.items64 = reinterpret_cast<unsigned short*>(sm + off[11]);
+  s.pitch = a.max_slots_pad;
   return s;
+}
+
+// What a visit of precision mode needs beyond its block: whether every update runs in
+// FP64, and the polish's rule for a settled vertex.
+struct PrecMode {
+  int f64_all, polish;
+};
+// Precision mode, behind load_visit3d and a CTA barrier: the slots' FP64 products and the
+// bounds that belong to their updates.
+__device__ __forceinline__ void load_prec3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, PrecMode pm) {
+  for (int j = threadIdx.x; j < bd.nslots; j += blockDim.x) {
+    const int f = a.slot_f64[bd.slot_begin + j];
+    s.sf[j] = f;
+    if (f >= 0) s.hs[j] = a.hs64[f];
+    else if (pm.f64_all) s.hs[j] = a.hsu64[bd.slot_begin + j];
+  }
+}
+
+// The FP64 updates of the apexes in `mask` (one bit each) of a slot with corner times T
+// and the products g; the others' times come back as they are.
+__device__ __noinline__ float4 slot_updates_f64(unsigned mask, float TA, float TB, float TC, float TD, double g0,
+                                                double g1, double g2, double g3, double g4, double g5) {
+  const double dACBC = g0, dBCCD = g1, dACCD = g2, dADBD = g3, dACAD = g4, dBCBD = g5;
+  const double dADBC = dACBC + dBCCD, dACBD = dACBC + dACCD;
+  const double dCDBD = dADBD - dACBD, dADCD = dADBD - dADBC;
+  const double dCDCD = dADCD - dACCD, dADAD = dADCD + dACAD, dACAC = dACAD - dACCD;
+  const double dBDBD = dBCBD + dCDBD, dBCBC = dBCBD - dBCCD;
+  const double A = (double)TA, B = (double)TB, C = (double)TC, D = (double)TD;
+  float4 r = make_float4(TA, TB, TC, TD);
+  if (mask & 8u) r.w = fminf(TD, w_float(tet_update_wide<PrecWide>(A, B, C, dACAC, dACBC, dACCD, dBCBC, dBCCD, dCDCD)));
+  if (mask & 1u) r.x = fminf(TA, w_float(tet_update_wide<PrecWide>(B, D, C, dBCBC, -dBCCD, -dACBC, dCDCD, dACCD, dACAC)));
+  if (mask & 2u) r.y = fminf(TB, w_float(tet_update_wide<PrecWide>(A, D, C, dACAC, -dACCD, -dACBC, dCDCD, dBCCD, dBCBC)));
+  if (mask & 4u) r.z = fminf(TC, w_float(tet_update_wide<PrecWide>(A, B, D, dADAD, dADBD, -dADCD, dBDBD, -dCDBD, dCDCD)));
+  return r;
 }
 
 // Loads block bd: the bulk copies of its coefficients, corner ids, bounds and `memo`
@@ -139,15 +184,68 @@ __device__ __forceinline__ void append_items(unsigned short* items, int* count, 
   if (need & 8u) items[base + n2 + __popc(bal[3] & below)] = (unsigned short)(4 * j + 3);
 }
 
+// Precision mode: appends slot j to the FP64 lists of the apex kinds in `need`; counts in
+// n[0..3].  All lanes of a warp together.
+__device__ __forceinline__ void append_items64(const SmemV& s, int* n, unsigned need, int j) {
+  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const unsigned bal = __ballot_sync(0xffffffffu, (need >> k) & 1u);
+    if (!bal) continue;
+    int base = 0;
+    if (lane == 0) base = atomicAdd(n + k, __popc(bal));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if ((need >> k) & 1u) s.items64[k * s.pitch + base + __popc(bal & below)] = (unsigned short)j;
+  }
+}
+template <bool kPrec>
+__device__ __forceinline__ void append_updates(const SmemV& s, int* s_n, PrecMode pm, unsigned need, int j) {
+  if constexpr (kPrec) {
+    const bool wide = need && (pm.f64_all || s.sf[j] >= 0);
+    append_items(s.items, s_n, wide ? 0u : need, j);
+    append_items64(s, s_n + 2, wide ? need : 0u, j);
+  } else {
+    append_items(s.items, s_n, need, j);
+  }
+}
+// counters of a visit: items, deferred slots, FP64 items per apex kind
+template <bool kPrec>
+__device__ __forceinline__ void clear_updates(int* s_n) {
+  if (threadIdx.x == 0) s_n[0] = 0;
+  if (kPrec && threadIdx.x < 4) s_n[2 + threadIdx.x] = 0;
+}
+
 // Runs the listed updates.  kPhase 0: the first sweep's owned apexes (into v1; *moved set
 // when one falls by EPS or more); 1: second-sweep owned apexes of slots whose copies are
 // known to keep their values (into v2), and first-sweep copies (into h0); 2: second-sweep
 // owned apexes of the slots whose copies phase 1 updated (into v2).
-template <int kPhase>
-__device__ __forceinline__ void run_items(const BlockDesc& bd, const SmemV& s, int count, volatile int* moved) {
-  const int nown = bd.nowned, pitch = bd.nslots_pad;
-  for (int i = threadIdx.x; i < count; i += blockDim.x) {
-    const int e = s.items[i], j = e >> 2, k = e & 3;
+template <int kPhase, bool kPrec>
+__device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd, const SmemV& s, const int* s_n,
+                                          volatile int* moved, PrecMode pm) {
+  const int nown = bd.nowned, pitch = bd.nslots_pad, lane = threadIdx.x & 31;
+  const int count = s_n[0], n32 = (count + 31) >> 5;
+  int n64 = 0, m0 = 0, m1 = 0, m2 = 0;
+  if constexpr (kPrec) {
+    m0 = (s_n[2] + 31) >> 5;
+    m1 = m0 + ((s_n[3] + 31) >> 5);
+    m2 = m1 + ((s_n[4] + 31) >> 5);
+    n64 = m2 + ((s_n[5] + 31) >> 5);
+  }
+  for (int c = threadIdx.x >> 5; c < n64 + n32; c += blockDim.x >> 5) {
+    int j, k;
+    const bool wide = kPrec && c < n64;
+    if (wide) {
+      k = (c >= m0) + (c >= m1) + (c >= m2);
+      const int r = ((c - (k == 0 ? 0 : k == 1 ? m0 : k == 2 ? m1 : m2)) << 5) + lane;
+      if (r >= s_n[2 + k]) continue;
+      j = s.items64[k * s.pitch + r];
+    } else {
+      const int r = ((c - n64) << 5) + lane;
+      if (r >= count) continue;
+      const int e = s.items[r];
+      j = e >> 2;
+      k = e & 3;
+    }
     int id[4];
     slot_ids(s.lv[j], id);
     const int idk = k < 2 ? (k == 0 ? id[0] : id[1]) : (k == 2 ? id[2] : id[3]);
@@ -164,15 +262,25 @@ __device__ __forceinline__ void run_items(const BlockDesc& bd, const SmemV& s, i
         T[q] = (kPhase == 1 && ownk && id[q] < nown) ? __int_as_float(s.v1[id[q]]) : s.vt[id[q]];
     }
     const float Tk = k < 2 ? (k == 0 ? T[0] : T[1]) : (k == 2 ? T[2] : T[3]);
-    const float* c = s.coef + j;
-    const TetGram g = tet_gram9(c[0], c[pitch], c[2 * pitch], c[3 * pitch], c[4 * pitch], c[5 * pitch]);
-    const float u = apex_update(k, T, g);
+    const float* cf = s.coef + j;
+    float u;
+    if (kPrec && wide) {
+      const int f = s.sf[j];
+      double g[6];
+#pragma unroll
+      for (int q = 0; q < 6; ++q) g[q] = (f >= 0) ? a.coef64[6 * (size_t)f + q] : (double)cf[q * pitch];
+      const float4 r = slot_updates_f64(1u << k, T[0], T[1], T[2], T[3], g[0], g[1], g[2], g[3], g[4], g[5]);
+      u = k < 2 ? (k == 0 ? r.x : r.y) : (k == 2 ? r.z : r.w);
+    } else {
+      const TetGram g = tet_gram9(cf[0], cf[pitch], cf[2 * pitch], cf[3 * pitch], cf[4 * pitch], cf[5 * pitch]);
+      u = apex_update(k, T, g);
+    }
     if (kPhase == 1 && !ownk) {
       reinterpret_cast<float*>(s.h0 + j)[k] = fminf(Tk, u);
     } else if (u < Tk) {
       atomicMin(kPhase == 0 ? &s.v1[idk] : &s.v2[idk], __float_as_int(u));
       // (double)(old - candidate) >= 1e-5 in the reference's check
-      if (kPhase == 0 && moved && !((Tk - u) <= kEps3DLe)) *moved = 1;
+      if (kPhase == 0 && moved && !((Tk - u) <= settle_eps(Tk, kPrec ? pm.polish : 0))) *moved = 1;
     }
   }
 }
@@ -180,9 +288,9 @@ __device__ __forceinline__ void run_items(const BlockDesc& bd, const SmemV& s, i
 // One check of a loaded block (its check memos in h0): whether it moves.  s_n: two
 // counters, zero on entry and on return.  All threads; ends behind a CTA barrier.
 // `aside` runs in the CTA's last warp while the others update: the items seldom reach it.
-template <class Aside>
+template <bool kPrec = false, class Aside>
 __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, int* s_n,
-                                              volatile int* s_moved, Aside aside) {
+                                              volatile int* s_moved, Aside aside, PrecMode pm = PrecMode{0, 0}) {
   const int tid = threadIdx.x, NT = blockDim.x, ns = bd.nslots, nown = bd.nowned;
   if (tid == 0) *s_moved = 0;
   for (int j0 = 0; j0 < ns; j0 += NT) {
@@ -205,14 +313,14 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
           need |= (id[k] < nown && m[k] < kLarge3DDev && !plane_skip(T[k], m[k], hs[k]) ? 1u : 0u) << k;
       }
     }
-    append_items(s.items, s_n, need, j);
+    append_updates<kPrec>(s, s_n, pm, need, j);
   }
   __syncthreads();
   if (tid >= NT - 32) aside();
-  run_items<0>(bd, s, s_n[0], s_moved);
+  run_items<0, kPrec>(a, bd, s, s_n, s_moved, pm);
   __syncthreads();
   const bool moved = *s_moved != 0;
-  if (tid == 0) s_n[0] = 0;
+  clear_updates<kPrec>(s_n);
   if (!moved)  // every slot's input times lowered no owned vertex by EPS
     for (int j = tid; j < ns; j += NT) {
       if (s.fl[j]) continue;
@@ -228,9 +336,9 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
 // The two sweeps of a loaded block (its sweep memos in h0, or behind a check read from
 // memory, where `memo` says they are of this solve): the final owned times in v2, those after the first sweep in v1.  s_n as above.
 // Ends behind a CTA barrier.
-template <class Aside>
+template <bool kPrec = false, class Aside>
 __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, int* s_n,
-                                              bool checked, bool memo, Aside aside) {
+                                              bool checked, bool memo, Aside aside, PrecMode pm = PrecMode{0, 0}) {
   const int tid = threadIdx.x, NT = blockDim.x, ns = bd.nslots, nown = bd.nowned;
   // ---- first sweep: owned apexes; bounds of the copies ----
   for (int j0 = 0; j0 < ns; j0 += NT) {
@@ -262,13 +370,13 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
       s.fl[j] = (unsigned char)(live & ~own);
       s.h0[j] = make_float4(lo[0], lo[1], lo[2], lo[3]);
     }
-    append_items(s.items, s_n, need, j);
+    append_updates<kPrec>(s, s_n, pm, need, j);
   }
   __syncthreads();
-  run_items<0>(bd, s, s_n[0], nullptr);
+  run_items<0, kPrec>(a, bd, s, s_n, nullptr, pm);
   __syncthreads();
   // ---- second sweep: owned apexes that the copies' bounds do not settle ----
-  if (tid == 0) s_n[0] = 0;
+  clear_updates<kPrec>(s_n);
   __syncthreads();
   for (int k = tid; k < nown; k += NT) s.v2[k] = s.v1[k];
   for (int j0 = 0; j0 < ns; j0 += NT) {
@@ -307,7 +415,7 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
             (unk & 4u) ? ~0u : __float_as_uint(T[2]), (unk & 8u) ? ~0u : __float_as_uint(T[3]));
       }
     }
-    append_items(s.items, s_n, need, j);
+    append_updates<kPrec>(s, s_n, pm, need, j);
     const unsigned bal = __ballot_sync(0xffffffffu, put);
     if (bal) {
       const unsigned lane = tid & 31u;
@@ -319,10 +427,10 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
   }
   __syncthreads();
   if (tid >= NT - 32) aside();
-  run_items<1>(bd, s, s_n[0], nullptr);
+  run_items<1, kPrec>(a, bd, s, s_n, nullptr, pm);
   __syncthreads();
   const int nd = s_n[1];
-  if (tid == 0) s_n[0] = 0;
+  clear_updates<kPrec>(s_n);
   if (nd > 0) {  // uniform across the CTA
     __syncthreads();
     for (int i0 = 0; i0 < nd; i0 += NT) {
@@ -352,11 +460,12 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
           a.fim_memo[bd.slot_begin + j] = make_uint4(__float_as_uint(T[0]), __float_as_uint(T[1]),
                                                      __float_as_uint(T[2]), __float_as_uint(T[3]));
       }
-      append_items(s.items, s_n, need, j);
+      append_updates<kPrec>(s, s_n, pm, need, j);
     }
     __syncthreads();
-    run_items<2>(bd, s, s_n[0], nullptr);
+    run_items<2, kPrec>(a, bd, s, s_n, nullptr, pm);
     __syncthreads();
-    if (tid == 0) s_n[0] = s_n[1] = 0;
+    clear_updates<kPrec>(s_n);
+    if (tid == 0) s_n[1] = 0;
   }
 }
