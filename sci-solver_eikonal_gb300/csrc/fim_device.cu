@@ -1288,7 +1288,10 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
   const int stamp = iter + 1;
   const int nact = ctl->nact;
   const int* cand = a.cand + (size_t)((iter + 1) & 1) * a.nb;
-  const int count = nact + ctl->ncand[(iter + 1) & 1];
+  const int ncand = ctl->ncand[(iter + 1) & 1], count = nact + ncand;
+  // with more active blocks than CTAs the candidates come first, so that the sweeps, all
+  // alike, end the launch (see k_loop3d)
+  const bool early = nact > (int)gridDim.x;
   int* list = act_list(a, iter);
   const PrecMode pm = kPrec ? PrecMode{ctl->f64_all, ctl->polish} : PrecMode{0, 0};
   stamp_start(a, iter, 0);
@@ -1303,8 +1306,8 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
   // spares every visit the instance lookup
   const int done1 = (a.ninst == 1) ? a.inst_done[0] : -1;
   while (item < count) {
-    const bool chk = item >= nact;  // a check candidate
-    const int b = chk ? cand[item - nact] : list[item];
+    const bool chk = early ? item < ncand : item >= nact;  // a check candidate
+    const int b = early ? (chk ? cand[item] : list[item - ncand]) : (chk ? cand[item - nact] : list[item]);
     const BlockDesc bd = a.blocks[b];
     // instance finished: leave its blocks alone; at its cap: its checks only
     const int ist = done1 >= 0 ? done1 : a.inst_done[a.blk_inst[b]];
