@@ -236,6 +236,12 @@ constexpr int kKStride = 16;    // words of per-iteration telemetry (DevArgs::kt
 #ifndef EIK_ITEM_MAXNREG
 #define EIK_ITEM_MAXNREG 56
 #endif
+#ifndef EIK_SPLIT4
+#define EIK_SPLIT4 1
+#endif
+#ifndef EIK_SPLIT2
+#define EIK_SPLIT2 1
+#endif
 #ifndef EIK_PREC_THREADS
 #define EIK_PREC_THREADS 384
 #endif

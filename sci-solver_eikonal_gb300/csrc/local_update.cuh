@@ -384,18 +384,25 @@ __device__ __forceinline__ float tet_inner_root(const TetInner& o, bool minus, A
   return fminf(kLarge3DDev, __fadd_rn(__fmaf_rn(TC, l3, __fmaf_rn(TA, l1, __fmul_rn(TB, l2))),
                                       __fsqrt_rn(x_dist3(f, l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
 }
-// The whole update of apex k's argument order; out of line, one body for all apex kinds,
-// which spares the instruction cache and lets a warp's lanes update different apexes.
-__device__ __noinline__ float tet_update_whole(int k, float TA, float TB, float TC, float ACAC, float ACBC, float ACCD,
-                                               float BCBC, float BCCD, float CDCD) {
+// The update of apex k's argument order, or its least candidate among `parts` (uniform
+// across a warp: bits 0 edge BC, 1 edge AC, 2 edge AB, 3 and 4 the inner roots with
+// +sqrt and -sqrt); out of line, one body for all apex kinds, which spares the
+// instruction cache and lets a warp's lanes update different apexes.
+constexpr unsigned kAllParts = 31u;
+__device__ __noinline__ float tet_update_parts(unsigned parts, int k, float TA, float TB, float TC, float ACAC,
+                                               float ACBC, float ACCD, float BCBC, float BCCD, float CDCD) {
   if (TA >= kLarge3DDev && TB >= kLarge3DDev && TC >= kLarge3DDev) return kLarge3DDev;
   const ApexFuse f = apex_fuse(k);
-  float best = fminf(tet_part_edge(false, f, TB, TC, BCBC, BCCD, CDCD), tet_part_edge(true, f, TA, TC, ACAC, ACCD, CDCD));
-  best = fminf(best, tet_part_ab(f, TA, TB, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
-  const TetInner o = tet_inner_setup(f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
-  if (o.sd >= 0.0f) {
-    best = fminf(best, tet_inner_root(o, false, f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
-    best = fminf(best, tet_inner_root(o, true, f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+  float best = kLarge3DDev;
+  if (parts & 1u) best = tet_part_edge(false, f, TB, TC, BCBC, BCCD, CDCD);
+  if (parts & 2u) best = fminf(best, tet_part_edge(true, f, TA, TC, ACAC, ACCD, CDCD));
+  if (parts & 4u) best = fminf(best, tet_part_ab(f, TA, TB, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+  if (parts & 24u) {
+    const TetInner o = tet_inner_setup(f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
+    if (o.sd >= 0.0f) {
+      if (parts & 8u) best = fminf(best, tet_inner_root(o, false, f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+      if (parts & 16u) best = fminf(best, tet_inner_root(o, true, f, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+    }
   }
   return best;
 }
@@ -426,9 +433,9 @@ __device__ __forceinline__ TetGram tet_gram9(float ACBC, float BCCD, float ACCD,
 // An apex update's arguments: the times of its face's corners and the metric products
 // as the reference passes them for apex k (0..3 = A, B, C, D).  k may differ between the
 // lanes of a warp: every argument is picked by selects.
-__device__ __forceinline__ float apex_update(int k, const float T[4], const TetGram& g) {
+__device__ __forceinline__ float apex_update(int k, const float T[4], const TetGram& g, unsigned parts = kAllParts) {
   const bool a = k == 0, c = k == 2, ab = k < 2;
-  return tet_update_whole(k, a ? T[1] : T[0], ab ? T[3] : T[1], c ? T[3] : T[2], a ? g.BCBC : c ? g.ADAD : g.ACAC,
+  return tet_update_parts(parts, k, a ? T[1] : T[0], ab ? T[3] : T[1], c ? T[3] : T[2], a ? g.BCBC : c ? g.ADAD : g.ACAC,
                           a ? -g.BCCD : c ? g.ADBD : ab ? -g.ACCD : g.ACBC, ab ? -g.ACBC : c ? -g.ADCD : g.ACCD,
                           ab ? g.CDCD : c ? g.BDBD : g.BCBC, a ? g.ACCD : c ? -g.CDBD : g.BCCD,
                           a ? g.ACAC : ab ? g.BCBC : g.CDCD);

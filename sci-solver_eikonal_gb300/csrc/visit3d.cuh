@@ -231,7 +231,11 @@ __device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd,
     m2 = m1 + ((s_n[4] + 31) >> 5);
     n64 = m2 + ((s_n[5] + 31) >> 5);
   }
-  for (int c = threadIdx.x >> 5; c < n64 + n32; c += blockDim.x >> 5) {
+  // Few chunks leave warps idle while each runs the long chain of a whole update: its
+  // parts then run side by side in two or four warps (their least is the update).
+  const int nw = blockDim.x >> 5;
+  const int split = n32 * 4 <= nw * EIK_SPLIT4 ? 2 : n32 * 2 <= nw * EIK_SPLIT2 ? 1 : 0;  // log2 of the parts
+  for (int c = threadIdx.x >> 5; c < n64 + (n32 << split); c += nw) {
     int j, k;
     const bool wide = kPrec && c < n64;
     if (wide) {
@@ -240,7 +244,7 @@ __device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd,
       if (r >= s_n[2 + k]) continue;
       j = s.items64[k * s.pitch + r];
     } else {
-      const int r = ((c - n64) << 5) + lane;
+      const int r = (((c - n64) >> split) << 5) + lane;
       if (r >= count) continue;
       const int e = s.items[r];
       j = e >> 2;
@@ -273,10 +277,14 @@ __device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd,
       u = k < 2 ? (k == 0 ? r.x : r.y) : (k == 2 ? r.z : r.w);
     } else {
       const TetGram g = tet_gram9(cf[0], cf[pitch], cf[2 * pitch], cf[3 * pitch], cf[4 * pitch], cf[5 * pitch]);
-      u = apex_update(k, T, g);
+      const int part = (c - n64) & ((1 << split) - 1);
+      const unsigned parts = split == 0 ? kAllParts : split == 1 ? (part ? 24u : 7u)
+                                                    : (part == 0 ? 8u : part == 1 ? 16u : part == 2 ? 4u : 3u);
+      u = apex_update(k, T, g, parts);
     }
     if (kPhase == 1 && !ownk) {
-      reinterpret_cast<float*>(s.h0 + j)[k] = fminf(Tk, u);
+      // (its place holds the copy's present value)
+      if (u < Tk) atomicMin(reinterpret_cast<int*>(s.h0 + j) + k, __float_as_int(u));
     } else if (u < Tk) {
       atomicMin(kPhase == 0 ? &s.v1[idk] : &s.v2[idk], __float_as_int(u));
       // (double)(old - candidate) >= 1e-5 in the reference's check
@@ -407,8 +415,11 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
                      : 0u)
                 << k;
       if (unk && need) {
-        need = unk;  // its copies first
+        need = unk;  // its copies first, from their present values
         put = true;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if ((unk >> q) & 1u) reinterpret_cast<float*>(s.h0 + j)[q] = s.vt[id[q]];
       } else if (a.fim_memo) {
         a.fim_memo[bd.slot_begin + j] = make_uint4(
             (unk & 1u) ? ~0u : __float_as_uint(T[0]), (unk & 2u) ? ~0u : __float_as_uint(T[1]),
