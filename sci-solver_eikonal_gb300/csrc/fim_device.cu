@@ -236,15 +236,6 @@ constexpr int kKStride = 16;    // words of per-iteration telemetry (DevArgs::kt
 #ifndef EIK_ITEM_MAXNREG
 #define EIK_ITEM_MAXNREG 56
 #endif
-#ifndef EIK_SPLIT4
-#define EIK_SPLIT4 1
-#endif
-#ifndef EIK_SPLIT2
-#define EIK_SPLIT2 1
-#endif
-#ifndef EIK_PREC_THREADS
-#define EIK_PREC_THREADS 384
-#endif
 #ifndef EIK_PREC_MAXNREG
 #define EIK_PREC_MAXNREG 80
 #endif
@@ -2500,6 +2491,18 @@ cudaError_t raise_smem_limit(const void* func, size_t bytes) {
 // CTA size of the item sweep and check kernels when the caller gives none
 constexpr int kItemThreads = EIK_ITEM_THREADS;
 
+// CTA size of the 3D loop kernel and of precision mode's item visits when the caller
+// gives none.  A mesh's blocks are active a fraction at a time: while fewer are than the
+// GPU holds CTAs, more warps per visit shorten it; when they fill the GPU, three visits
+// per SM overlap better.  Solves on one GB300 in us at 384 / 512 / 768 threads (three, two
+// and one CTA per SM): 562 blocks 1088 / 969 / 948, 792 blocks 1338 / 1238 / 1188, 1077
+// blocks 1482 / 1392 / 1414, 2894 blocks 2826 / 2733 / 3121, 4292 blocks 3156 / 3186 /
+// 4014.
+int items_threads(int nb, int nsm, bool prec) {
+  if (nb <= 6 * nsm) return 768;
+  return (nb <= 24 * nsm && !prec) ? 512 : kItemThreads;
+}
+
 // Precision mode's polish: rounds, iterations per round, and the relative gap
 // between a vertex's time and its FP64 update above which its block runs again.
 constexpr int kPolishRounds = 8;
@@ -2852,10 +2855,13 @@ std::string DeviceSolve::Impl::run_loop3d(const Layout& L, const SolveOptions& o
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     P.loop_smem = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, false);
-    CK(raise_smem_limit((const void*)k_loop3d, P.loop_smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_loop3d, threads, P.loop_smem));
+    // as many registers as the CTAs that shared memory lets an SM hold leave
+    const void* f = threads <= 384 ? (const void*)k_loop3d<56> : threads <= 512 ? (const void*)k_loop3d<64>
+                    : threads <= 768 ? (const void*)k_loop3d<80> : (const void*)k_loop3d<64>;
+    CK(raise_smem_limit(f, P.loop_smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads, P.loop_smem));
     if (occ < 1) return "loop kernel cannot be resident (shared memory / registers)";
-    P.loop_func = (const void*)k_loop3d;
+    P.loop_func = f;
     P.loop_threads = threads;
     P.loop_grid = std::max(1, std::min(occ * nsm, L.nb));
   }
@@ -3494,7 +3500,7 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
     // (65^3 workload: solve 7.85 ms against 7.93 at 512 and 8.4 at one thread per slot)
     threads = kItemThreads;
   } else if (!given && items64) {
-    threads = EIK_PREC_THREADS;
+    threads = kItemThreads;
   } else if (!given && L.dim == 3) {
     const int full = threads, half = auto_visit_threads(P.max_slots_pad);
     if (half < full) {
@@ -3512,6 +3518,12 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   const bool loop2d = L.dim == 2 && sweeps == 7 && !opt.direct_launch && P.max_slots_pad <= 1024;
   // 3D ones of its two sweeps in another (k_loop3d)
   const bool loop3d = L.dim == 3 && items && sweeps == 2 && !opt.direct_launch;
+  if (!given && (loop3d || items64)) {
+    int dev = 0, nsm = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    threads = items_threads(L.nb, nsm, P.prec);
+  }
   // per-instance iteration caps (one cap for all when not given)
   std::vector<int> cap(P.ninst, opt.max_iterations);
   if ((int)opt.inst_max_iterations.size() == P.ninst) cap = opt.inst_max_iterations;

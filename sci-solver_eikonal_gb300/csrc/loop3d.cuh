@@ -166,7 +166,8 @@ __device__ __forceinline__ void next_item(const DevArgs& a, const Start3& st, co
   }
 }
 
-__global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_loop3d(const __grid_constant__ DevArgs a,
+template <int kRegs>
+__global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
                                                                  const __grid_constant__ Start3 st) {
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ __align__(8) unsigned long long bar;

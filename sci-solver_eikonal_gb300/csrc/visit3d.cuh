@@ -234,7 +234,7 @@ __device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd,
   // Few chunks leave warps idle while each runs the long chain of a whole update: its
   // parts then run side by side in two or four warps (their least is the update).
   const int nw = blockDim.x >> 5;
-  const int split = n32 * 4 <= nw * EIK_SPLIT4 ? 2 : n32 * 2 <= nw * EIK_SPLIT2 ? 1 : 0;  // log2 of the parts
+  const int split = n32 * 4 <= nw ? 2 : n32 * 2 <= nw ? 1 : 0;  // log2 of the parts
   for (int c = threadIdx.x >> 5; c < n64 + (n32 << split); c += nw) {
     int j, k;
     const bool wide = kPrec && c < n64;
