@@ -268,13 +268,25 @@ void tet_gram(const float* xyz, const int* t, const float* m, float g[6]) {
   g[5] = uMw(BC, BD);
 }
 
+// Smallest and largest index in one pass that the compiler can vectorise (two passes with
+// early exits took 1 ms of a 33^3 cube's hand-over).
+__attribute__((optimize("O3"))) static void index_range(const int* e, size_t n, int* mn, int* mx) {
+  int lo = e[0], hi = e[0];
+  for (size_t i = 0; i < n; ++i) {
+    lo = e[i] < lo ? e[i] : lo;
+    hi = e[i] > hi ? e[i] : hi;
+  }
+  *mn = lo;
+  *mx = hi;
+}
+
 std::string normalize_index_base(std::vector<int>& e, int nv) {
   if (e.empty()) return "no elements";
-  const int mn = *std::min_element(e.begin(), e.end());
+  int mn, mx;
+  index_range(e.data(), e.size(), &mn, &mx);
   if (mn == 1) for (int& x : e) x -= 1;
   else if (mn != 0) return "element indices must start from 0 or 1";
-  for (int x : e)
-    if (x < 0 || x >= nv) return "element index out of range";
+  if ((long long)mx - mn >= nv) return "element index out of range";
   return "";
 }
 
@@ -323,7 +335,8 @@ void rcb(RcbPoint* p, int n, int nparts, int first, int* labels, int depth) {
     return a.c[ax] < b.c[ax] || (a.c[ax] == b.c[ax] && a.id < b.id);
   });
   // the two halves are independent: the first levels run them on two threads
-  if (depth < 4 && n >= 32768) {
+  // (a thread takes about 20 us to start, 4096 points about 100 us to split up)
+  if (depth < 4 && n >= 4096) {
     std::thread left([=] { rcb(p, nl, pl, first, labels, depth + 1); });
     rcb(p + nl, n - nl, nparts - pl, first + pl, labels, depth + 1);
     left.join();
