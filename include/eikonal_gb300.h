@@ -244,7 +244,10 @@ int eik_tri_prep_values(const eik_solver* h, float* edges, float* speed_inv, flo
  *   which = 6: the four apex updates of one slot as the 3D visit kernels run them
  *              (FIMCuda's group, CUDA_kernels.cu:454-457, with its roundings), 10
  *              inputs per case (TA TB TC TD, then the stored products ACBC BCCD ACCD
- *              ADBD ACAD BCBD), 4 outputs min(T_k, update of apex k). */
+ *              ADBD ACAD BCBD), 4 outputs min(T_k, update of apex k).
+ *   which = 7: the same of precision mode's FP64 updates, from products given in
+ *   FP32.
+ */
 int eik_selftest_local_update(int which, const float* in, float* out, int n);
 
 /* Failure-path self-test (no counterpart in the reference, which has no bounded

@@ -1277,7 +1277,7 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int s_item;
-  __shared__ int s_n[6];
+  __shared__ int s_n[3];
   __shared__ volatile int s_moved;
   const SmemV s = carve_visit3d<kPrec>(sm, a);
   const int tid = threadIdx.x, NT = blockDim.x;
@@ -1294,7 +1294,7 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
   const PrecMode pm = kPrec ? PrecMode{ctl->f64_all, ctl->polish} : PrecMode{0, 0};
   stamp_start(a, iter, 0);
   if (tid == 0) mbar_init(&bar, 1);
-  if (tid < 6) s_n[tid] = 0;
+  if (tid < 3) s_n[tid] = 0;
   __syncthreads();
   unsigned parity = 0;
   // the first block of a CTA is its own index; later ones come from the counter
@@ -2442,6 +2442,16 @@ __global__ void k_selftest_tet_group(const float* in, float* out, int n) {
     o[1] = fminf(T[1], apex_update(1, T, g));
     o[2] = fminf(T[2], apex_update(2, T, g));
     o[3] = fminf(T[3], apex_update(3, T, g));
+  }
+}
+// the same for precision mode's FP64 updates, from products given in FP32
+__global__ void k_selftest_tet64_group(const float* in, float* out, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    const float* a = in + 10 * (size_t)i;
+    const float T[4] = {a[0], a[1], a[2], a[3]};
+    const double g[6] = {a[4], a[5], a[6], a[7], a[8], a[9]};
+    for (int k = 0; k < 4; ++k) out[4 * (size_t)i + k] = fminf(T[k], apex_update64(k, T, g));
   }
 }
 __global__ void k_selftest_tri(const float* in, float* out, int n) {
@@ -4173,8 +4183,8 @@ std::string selftest_wait_timeout(int* status, double* waited_ms) {
 
 std::string selftest_device(int which, const float* in, float* out, int n) {
   if (which == 3 || which == 4) return selftest_tri_blocks(in, n, which == 4, out);
-  const int nin = (which == 0 || which == 5) ? 9 : (which == 1) ? 7 : (which == 6) ? 10 : 2;
-  const int nout = (which == 2) ? 2 : (which == 6) ? 4 : 1;
+  const int nin = (which == 0 || which == 5) ? 9 : (which == 1) ? 7 : (which >= 6) ? 10 : 2;
+  const int nout = (which == 2) ? 2 : (which >= 6) ? 4 : 1;
   float *din = nullptr, *dout = nullptr;
   CK(cudaMalloc((void**)&din, sizeof(float) * (size_t)nin * n + 16));
   CK(cudaMalloc((void**)&dout, sizeof(float) * (size_t)nout * n + 16));
@@ -4185,6 +4195,7 @@ std::string selftest_device(int which, const float* in, float* out, int n) {
     else if (which == 5) k_selftest_tet64<<<grid, 128>>>(din, dout, n);
     else if (which == 1) k_selftest_tri<<<grid, 128>>>(din, dout, n);
     else if (which == 6) k_selftest_tet_group<<<grid, 128>>>(din, dout, n);
+    else if (which == 7) k_selftest_tet64_group<<<grid, 128>>>(din, dout, n);
     else k_selftest_quot<<<grid, 128>>>(din, dout, n);
   }
   cudaError_t e = cudaDeviceSynchronize();

@@ -558,6 +558,133 @@ __device__ __forceinline__ double tet_update_f64(double TA, double TB, double TC
   return tet_update_wide<double>(TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD);
 }
 
+// The same update of apex k with its roundings written out: each fused multiply-add is
+// the one the compiler chose for tet_update_wide in the kernel that ran precision mode
+// before, so the results do not depend on the code around it.  The choice matters where
+// two corners' times nearly agree: p, q and r then cancel, and a discriminant's sign
+// decides whether a slab of the face counts at all.  One rule covers the four kinds (the
+// products of t and of BCCD's row are fused the other way round for A, B, C and for C);
+// it reproduces that kernel's bits on 512 000 updates, two thirds of them with two times
+// within 600 units in the last place.  One body for all kinds: the lanes of a warp
+// update different apexes.  `parts` as in tet_update_parts.
+__device__ __forceinline__ double d_ms(bool b, double x, double y, double z, double w) {  // x*y - z*w
+  const double pr = __dmul_rn(b ? x : z, b ? y : w);
+  return __fma_rn(b ? -z : x, b ? w : y, b ? pr : -pr);
+}
+__device__ __forceinline__ double d_root(double q, double sd, double i2p) { return __dmul_rn(__dadd_rn(-q, sd), i2p); }
+__device__ __forceinline__ double d_dist3(double l1, double l2, double ACAC, double ACBC, double ACCD, double BCBC,
+                                          double BCCD, double CDCD) {
+  const double X = __fma_rn(l1, ACAC, __fma_rn(l2, ACBC, ACCD)), Y = __fma_rn(l1, ACBC, __fma_rn(l2, BCBC, BCCD));
+  return __fma_rn(X, l1, __fma_rn(Y, l2, __fma_rn(l1, ACCD, __fma_rn(l2, BCCD, CDCD))));
+}
+// an edge XC of the face: its inner candidates and its end points
+__device__ __forceinline__ double tet64_part_edge(double TX, double TC, double XX, double XC, double CC) {
+  const double T = __dsub_rn(TC, TX), XC2 = __dadd_rn(XC, XC);
+  const double p = d_ms(false, __dmul_rn(XX, T), T, XX, XX);
+  const double q = d_ms(false, __dmul_rn(XC2, T), T, __dmul_rn(2.0, XX), XC);
+  const double r = d_ms(false, __dmul_rn(T, T), CC, XC, XC);
+  const double delta = d_ms(false, q, q, __dmul_rn(4.0, p), r);
+  double best = fmin(__dadd_rn(TX, sqrt_pos(__dadd_rn(__dadd_rn(XX, XC), __dadd_rn(XC, CC)))), __dadd_rn(TC, sqrt_pos(CC)));
+  best = fmin((double)kLarge3DDev, best);
+  if (delta >= 0.0) {
+    const double sd = __dsqrt_rn(delta), i2p = __drcp_rn(__dmul_rn(2.0, p));
+#pragma unroll 1
+    for (int sg = 0; sg < 2; ++sg) {
+      const double l = d_root(q, sg ? -sd : sd, i2p), m = __dsub_rn(1.0, l);
+      if (l >= 0 && l <= 1)
+        best = fmin(best, __dadd_rn(__fma_rn(TX, l, __dmul_rn(TC, m)),
+                                    sqrt_pos(__fma_rn(__fma_rn(l, XX, XC), l, __fma_rn(l, XC, CC)))));
+    }
+  }
+  return best;
+}
+// edge AB; its end points are candidates of the other two edges
+__device__ __forceinline__ double tet64_part_ab(double TA, double TB, double ACAC, double ACBC, double ACCD, double BCBC,
+                                                double BCCD, double CDCD) {
+  const double T = __dsub_rn(TB, TA), T2 = __dmul_rn(T, T);
+  const double gx = __dsub_rn(ACAC, ACBC), gy = __dsub_rn(ACBC, BCBC), gz = __dsub_rn(ACCD, BCCD);
+  const double P1 = d_ms(false, T2, ACAC, gx, gx), P2 = d_ms(false, __dmul_rn(BCBC, T), T, gy, gy);
+  const double P3 = d_ms(false, __dmul_rn(__dadd_rn(ACBC, ACBC), T), T, __dmul_rn(2.0, gx), gy);
+  const double P4 = d_ms(false, __dmul_rn(__dadd_rn(ACCD, ACCD), T), T, __dmul_rn(2.0, gx), gz);
+  const double P5 = d_ms(false, __dmul_rn(__dadd_rn(BCCD, BCCD), T), T, __dmul_rn(2.0, gy), gz);
+  const double p = __dsub_rn(__dadd_rn(P1, P2), P3);
+  const double q = __dsub_rn(__dadd_rn(__dadd_rn(__dmul_rn(-P2, 2.0), P3), P4), P5);
+  const double r = __dadd_rn(__dadd_rn(d_ms(false, T2, BCBC, gy, gy), P5), d_ms(false, T2, CDCD, gz, gz));
+  const double delta = d_ms(false, q, q, __dmul_rn(4.0, p), r);
+  double best = (double)kLarge3DDev;
+  if (delta >= 0.0) {
+    const double sd = __dsqrt_rn(delta), i2p = __drcp_rn(__dmul_rn(2.0, p));
+#pragma unroll 1
+    for (int sg = 0; sg < 2; ++sg) {
+      const double l1 = d_root(q, sg ? -sd : sd, i2p), l2 = __dsub_rn(1.0, l1);
+      if (l1 >= 0 && l1 <= 1) {
+        const double X = __dadd_rn(__fma_rn(l1, ACAC, __dmul_rn(l2, ACBC)), ACCD);
+        const double Y = __dadd_rn(__fma_rn(l1, ACBC, __dmul_rn(l2, BCBC)), BCCD);
+        const double Z = __dadd_rn(__fma_rn(l1, ACCD, __dmul_rn(l2, BCCD)), CDCD);
+        best = fmin(best, __dadd_rn(__fma_rn(TA, l1, __dmul_rn(TB, l2)),
+                                    sqrt_pos(__dadd_rn(__dadd_rn(__dmul_rn(X, l1), __dmul_rn(Y, l2)), Z))));
+      }
+    }
+  }
+  return best;
+}
+// inside the face: roots with +sqrt (parts bit 3) and -sqrt (bit 4)
+__device__ __forceinline__ double tet64_part_inner(unsigned parts, int k, double TA, double TB, double TC, double ACAC,
+                                                   double ACBC, double ACCD, double BCBC, double BCCD, double CDCD) {
+  const double TAC = __dsub_rn(TC, TA), TBC = __dsub_rn(TC, TB), TAC2 = __dmul_rn(TAC, TAC);
+  const double s = d_ms(false, TAC, ACBC, TBC, ACAC);
+  const double t = d_ms(k < 3, TAC, BCCD, TBC, ACCD);
+  const double h = -d_ms(true, TAC, BCBC, TBC, ACBC);
+  const double P1 = d_ms(false, TAC2, ACAC, ACAC, ACAC), P2 = d_ms(false, __dmul_rn(BCBC, TAC), TAC, ACBC, ACBC);
+  const double P3 = d_ms(false, __dmul_rn(__dadd_rn(ACBC, ACBC), TAC), TAC, __dmul_rn(2.0, ACAC), ACBC);
+  const double P4 = d_ms(false, __dmul_rn(__dadd_rn(ACCD, ACCD), TAC), TAC, __dmul_rn(2.0, ACAC), ACCD);
+  const double P5 = d_ms(k == 2, __dmul_rn(__dadd_rn(BCCD, BCCD), TAC), TAC, __dmul_rn(2.0, ACBC), ACCD);
+  const double P6 = d_ms(false, TAC2, BCBC, ACBC, ACBC), P7 = d_ms(false, TAC2, CDCD, ACCD, ACCD);
+  const double p = __fma_rn(__dmul_rn(P3, s), h, __fma_rn(__dmul_rn(P2, s), s, __dmul_rn(__dmul_rn(P1, h), h)));
+  double q = __fma_rn(__dmul_rn(__dmul_rn(P2, 2.0), s), t, __dmul_rn(__dmul_rn(P3, t), h));
+  q = __fma_rn(__dmul_rn(P5, s), h, __fma_rn(__dmul_rn(P4, h), h, q));
+  const double r =
+      __fma_rn(__dmul_rn(P7, h), h, __fma_rn(__dmul_rn(P6, t), t, __dmul_rn(__dmul_rn(P5, t), h)));
+  const double delta = d_ms(false, q, q, __dmul_rn(4.0, p), r);
+  double best = (double)kLarge3DDev;
+  if (delta >= 0.0) {
+    const double sd = __dsqrt_rn(delta), i2p = __drcp_rn(__dmul_rn(2.0, p)), ih = __drcp_rn(__dadd_rn(h, 0.00000001));
+#pragma unroll 1
+    for (int sg = 0; sg < 2; ++sg) {
+      if (!((parts >> (3 + sg)) & 1u)) continue;
+      const double l1 = d_root(q, sg ? -sd : sd, i2p), l2 = __dmul_rn(__fma_rn(s, l1, t), ih);
+      const double l3 = __dsub_rn(__dsub_rn(1.0, l1), l2);
+      if (l1 >= 0 && l1 <= 1 && l2 >= 0 && l2 <= 1 && l3 >= 0 && l3 <= 1)
+        best = fmin(best, __dadd_rn(__fma_rn(TC, l3, __fma_rn(TA, l1, __dmul_rn(TB, l2))),
+                                    sqrt_pos(d_dist3(l1, l2, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD))));
+    }
+  }
+  return best;
+}
+__device__ __noinline__ float tet64_update_parts(unsigned parts, int k, double TA, double TB, double TC, double ACAC,
+                                                 double ACBC, double ACCD, double BCBC, double BCCD, double CDCD) {
+  const double L = (double)kLarge3DDev;
+  if (TA >= L && TB >= L && TC >= L) return kLarge3DDev;
+  double best = L;
+  if (parts & 1u) best = tet64_part_edge(TB, TC, BCBC, BCCD, CDCD);
+  if (parts & 2u) best = fmin(best, tet64_part_edge(TA, TC, ACAC, ACCD, CDCD));
+  if (parts & 4u) best = fmin(best, tet64_part_ab(TA, TB, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+  if (parts & 24u) best = fmin(best, tet64_part_inner(parts, k, TA, TB, TC, ACAC, ACBC, ACCD, BCBC, BCCD, CDCD));
+  return (float)best;
+}
+// Apex k of a slot with corner times T and the six products g, as apex_update.
+__device__ __forceinline__ float apex_update64(int k, const float T[4], const double g[6], unsigned parts = kAllParts) {
+  const double ACBC = g[0], BCCD = g[1], ACCD = g[2], ADBD = g[3], ACAD = g[4], BCBD = g[5];
+  const double ADBC = __dadd_rn(ACBC, BCCD), ACBD = __dadd_rn(ACBC, ACCD);
+  const double CDBD = __dsub_rn(ADBD, ACBD), ADCD = __dsub_rn(ADBD, ADBC);
+  const double CDCD = __dsub_rn(ADCD, ACCD), ADAD = __dadd_rn(ADCD, ACAD), ACAC = __dsub_rn(ACAD, ACCD);
+  const double BDBD = __dadd_rn(BCBD, CDBD), BCBC = __dsub_rn(BCBD, BCCD);
+  const bool a = k == 0, c = k == 2, ab = k < 2;
+  return tet64_update_parts(parts, k, a ? T[1] : T[0], ab ? T[3] : T[1], c ? T[3] : T[2], a ? BCBC : c ? ADAD : ACAC,
+                            a ? -BCCD : c ? ADBD : ab ? -ACCD : ACBC, ab ? -ACBC : c ? -ADCD : ACCD,
+                            ab ? CDCD : c ? BDBD : BCBC, a ? ACCD : c ? -CDBD : BCCD, a ? ACAC : ab ? BCBC : CDCD);
+}
+
 // Triangle update of corner C from A and B; F is the inverse speed.  Uses the
 // reference's MIN macro semantics ((a)<(b)?(a):(b)), not fminf.
 __device__ __forceinline__ float mn2(float a, float b) { return (a < b) ? a : b; }

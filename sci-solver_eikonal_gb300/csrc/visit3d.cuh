@@ -34,34 +34,34 @@ struct SmemV {
   float* vt;              // owned times, then halo times
   int* v1;                // owned: bits of the times after the first sweep
   int* v2;                // ... after the second
-  unsigned short* items;  // 4 slot + apex, at most 4 per slot
+  unsigned short* items;  // 4 slot + apex, at most 4 per slot; precision mode: the FP64 updates from the end
   unsigned short* defer;  // slots whose copies the second sweep needs
   unsigned char* fl;      // per slot: copies of unknown value (bits 0-3), settled by the check memo (bit 7)
   int* sf;                // precision mode: per slot the FP64 products of its tet, or -1
-  unsigned short* items64;  // ... slots of the listed FP64 updates, one list of `pitch` per apex
-  int pitch;
 };
 // Precision mode (kPrec): the updates of flagged tets, and in the polish of all, run in
-// FP64.  They are listed apart, one list per apex kind, so that every FP64 instruction of
-// a warp works for all of its lanes: the FP64 unit takes 16 cycles for a warp whatever
-// the number of lanes in use, and it is what bounds the mode.
-__host__ __device__ inline size_t visit3d_offsets(int np, int max_local, int max_owned, bool prec, size_t off[12]) {
+// FP64.  They are listed apart, so that every FP64 instruction of a warp works for all of
+// its lanes: the FP64 unit takes 16 cycles for a warp whatever the number of lanes in
+// use, and it is what bounds the mode.  A 25^3 solve with slivers took 39.5 ms with an
+// update per slot, 13.0 ms with a list per apex kind, 11.2 ms with one list and body for
+// all kinds, split over idle warps like the FP32 updates.
+__host__ __device__ inline size_t visit3d_offsets(int np, int max_local, int max_owned, bool prec, size_t off[11]) {
   size_t o = 0;
-  const size_t n = (size_t)np, bytes[12] = {24 * n, 8 * n, 8 * n, 16 * n, 4 * (size_t)max_local, 4 * (size_t)max_owned,
-                                            4 * (size_t)max_owned, 8 * n, 2 * n, n, prec ? 4 * n : 0, prec ? 8 * n : 0};
-  for (int i = 0; i < 12; ++i) {
+  const size_t n = (size_t)np, bytes[11] = {24 * n, 8 * n, 8 * n, 16 * n, 4 * (size_t)max_local, 4 * (size_t)max_owned,
+                                            4 * (size_t)max_owned, 8 * n, 2 * n, n, prec ? 4 * n : 0};
+  for (int i = 0; i < 11; ++i) {
     off[i] = o;
     o += (bytes[i] + 15) & ~(size_t)15;
   }
   return o;
 }
 __host__ __device__ inline size_t smem_bytes_visit3d(int np, int max_local, int max_owned, bool prec) {
-  size_t off[12];
+  size_t off[11];
   return visit3d_offsets(np, max_local, max_owned, prec, off);
 }
 template <bool kPrec>
 __device__ __forceinline__ SmemV carve_visit3d(unsigned char* sm, const DevArgs& a) {
-  size_t off[12];
+  size_t off[11];
   visit3d_offsets(a.max_slots_pad, a.max_local, a.max_owned, kPrec, off);
   SmemV s;
   s.coef = reinterpret_cast<float*>(sm + off[0]);
@@ -75,8 +75,6 @@ __device__ __forceinline__ SmemV carve_visit3d(unsigned char* sm, const DevArgs&
   s.defer = reinterpret_cast<unsigned short*>(sm + off[8]);
   s.fl = sm + off[9];
   s.sf = reinterpret_cast<int*>(sm + off[10]);
-  s.items64 = reinterpret_cast<unsigned short*>(sm + off[11]);
-  s.pitch = a.max_slots_pad;
   return s;
 }
 
@@ -94,24 +92,6 @@ __device__ __forceinline__ void load_prec3d(const DevArgs& a, const BlockDesc& b
     if (f >= 0) s.hs[j] = a.hs64[f];
     else if (pm.f64_all) s.hs[j] = a.hsu64[bd.slot_begin + j];
   }
-}
-
-// The FP64 updates of the apexes in `mask` (one bit each) of a slot with corner times T
-// and the products g; the others' times come back as they are.
-__device__ __noinline__ float4 slot_updates_f64(unsigned mask, float TA, float TB, float TC, float TD, double g0,
-                                                double g1, double g2, double g3, double g4, double g5) {
-  const double dACBC = g0, dBCCD = g1, dACCD = g2, dADBD = g3, dACAD = g4, dBCBD = g5;
-  const double dADBC = dACBC + dBCCD, dACBD = dACBC + dACCD;
-  const double dCDBD = dADBD - dACBD, dADCD = dADBD - dADBC;
-  const double dCDCD = dADCD - dACCD, dADAD = dADCD + dACAD, dACAC = dACAD - dACCD;
-  const double dBDBD = dBCBD + dCDBD, dBCBC = dBCBD - dBCCD;
-  const double A = (double)TA, B = (double)TB, C = (double)TC, D = (double)TD;
-  float4 r = make_float4(TA, TB, TC, TD);
-  if (mask & 8u) r.w = fminf(TD, w_float(tet_update_wide<PrecWide>(A, B, C, dACAC, dACBC, dACCD, dBCBC, dBCCD, dCDCD)));
-  if (mask & 1u) r.x = fminf(TA, w_float(tet_update_wide<PrecWide>(B, D, C, dBCBC, -dBCCD, -dACBC, dCDCD, dACCD, dACAC)));
-  if (mask & 2u) r.y = fminf(TB, w_float(tet_update_wide<PrecWide>(A, D, C, dACAC, -dACCD, -dACBC, dCDCD, dBCCD, dBCBC)));
-  if (mask & 4u) r.z = fminf(TC, w_float(tet_update_wide<PrecWide>(A, B, D, dADAD, dADBD, -dADCD, dBDBD, -dCDBD, dCDCD)));
-  return r;
 }
 
 // Loads block bd: the bulk copies of its coefficients, corner ids, bounds and `memo`
@@ -167,7 +147,9 @@ __device__ __forceinline__ unsigned same_bits(const float T[4], uint4 m) {
   return (__float_as_uint(T[0]) == m.x ? 1u : 0u) | (__float_as_uint(T[1]) == m.y ? 2u : 0u) |
          (__float_as_uint(T[2]) == m.z ? 4u : 0u) | (__float_as_uint(T[3]) == m.w ? 8u : 0u);
 }
-// Appends slot j's apexes of `need` to the item list; all lanes of a warp together.
+// Appends slot j's apexes of `need` to the item list, which grows from `items` by kStep
+// entries at a time; all lanes of a warp together.
+template <int kStep = 1>
 __device__ __forceinline__ void append_items(unsigned short* items, int* count, unsigned need, int j) {
   const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   unsigned bal[4];
@@ -178,41 +160,28 @@ __device__ __forceinline__ void append_items(unsigned short* items, int* count, 
   int base = 0;
   if (lane == 0) base = atomicAdd(count, n);
   base = __shfl_sync(0xffffffffu, base, 0);
-  if (need & 1u) items[base + __popc(bal[0] & below)] = (unsigned short)(4 * j);
-  if (need & 2u) items[base + n0 + __popc(bal[1] & below)] = (unsigned short)(4 * j + 1);
-  if (need & 4u) items[base + n1 + __popc(bal[2] & below)] = (unsigned short)(4 * j + 2);
-  if (need & 8u) items[base + n2 + __popc(bal[3] & below)] = (unsigned short)(4 * j + 3);
-}
-
-// Precision mode: appends slot j to the FP64 lists of the apex kinds in `need`; counts in
-// n[0..3].  All lanes of a warp together.
-__device__ __forceinline__ void append_items64(const SmemV& s, int* n, unsigned need, int j) {
-  const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const unsigned bal = __ballot_sync(0xffffffffu, (need >> k) & 1u);
-    if (!bal) continue;
-    int base = 0;
-    if (lane == 0) base = atomicAdd(n + k, __popc(bal));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if ((need >> k) & 1u) s.items64[k * s.pitch + base + __popc(bal & below)] = (unsigned short)j;
-  }
+  if (need & 1u) items[kStep * (base + __popc(bal[0] & below))] = (unsigned short)(4 * j);
+  if (need & 2u) items[kStep * (base + n0 + __popc(bal[1] & below))] = (unsigned short)(4 * j + 1);
+  if (need & 4u) items[kStep * (base + n1 + __popc(bal[2] & below))] = (unsigned short)(4 * j + 2);
+  if (need & 8u) items[kStep * (base + n2 + __popc(bal[3] & below))] = (unsigned short)(4 * j + 3);
 }
 template <bool kPrec>
-__device__ __forceinline__ void append_updates(const SmemV& s, int* s_n, PrecMode pm, unsigned need, int j) {
+__device__ __forceinline__ void append_updates(const DevArgs& a, const SmemV& s, int* s_n, PrecMode pm, unsigned need,
+                                               int j) {
   if constexpr (kPrec) {
+    // an update is in one of the lists, so the two ends of the array never meet
     const bool wide = need && (pm.f64_all || s.sf[j] >= 0);
     append_items(s.items, s_n, wide ? 0u : need, j);
-    append_items64(s, s_n + 2, wide ? need : 0u, j);
+    append_items<-1>(s.items + 4 * a.max_slots_pad - 1, s_n + 2, wide ? need : 0u, j);
   } else {
     append_items(s.items, s_n, need, j);
   }
 }
-// counters of a visit: items, deferred slots, FP64 items per apex kind
+// counters of a visit: items, deferred slots, FP64 items
 template <bool kPrec>
 __device__ __forceinline__ void clear_updates(int* s_n) {
   if (threadIdx.x == 0) s_n[0] = 0;
-  if (kPrec && threadIdx.x < 4) s_n[2 + threadIdx.x] = 0;
+  if (kPrec && threadIdx.x == 0) s_n[2] = 0;
 }
 
 // Runs the listed updates.  kPhase 0: the first sweep's owned apexes (into v1; *moved set
@@ -224,32 +193,19 @@ __device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd,
                                           volatile int* moved, PrecMode pm) {
   const int nown = bd.nowned, pitch = bd.nslots_pad, lane = threadIdx.x & 31;
   const int count = s_n[0], n32 = (count + 31) >> 5;
-  int n64 = 0, m0 = 0, m1 = 0, m2 = 0;
-  if constexpr (kPrec) {
-    m0 = (s_n[2] + 31) >> 5;
-    m1 = m0 + ((s_n[3] + 31) >> 5);
-    m2 = m1 + ((s_n[4] + 31) >> 5);
-    n64 = m2 + ((s_n[5] + 31) >> 5);
-  }
+  const int count64 = kPrec ? s_n[2] : 0, n64 = (count64 + 31) >> 5;
   // Few chunks leave warps idle while each runs the long chain of a whole update: its
   // parts then run side by side in two or four warps (their least is the update).
   const int nw = blockDim.x >> 5;
-  const int split = n32 * 4 <= nw ? 2 : n32 * 2 <= nw ? 1 : 0;  // log2 of the parts
-  for (int c = threadIdx.x >> 5; c < n64 + (n32 << split); c += nw) {
-    int j, k;
-    const bool wide = kPrec && c < n64;
-    if (wide) {
-      k = (c >= m0) + (c >= m1) + (c >= m2);
-      const int r = ((c - (k == 0 ? 0 : k == 1 ? m0 : k == 2 ? m1 : m2)) << 5) + lane;
-      if (r >= s_n[2 + k]) continue;
-      j = s.items64[k * s.pitch + r];
-    } else {
-      const int r = (((c - n64) >> split) << 5) + lane;
-      if (r >= count) continue;
-      const int e = s.items[r];
-      j = e >> 2;
-      k = e & 3;
-    }
+  const int split = (n64 + n32) * 4 <= nw ? 2 : (n64 + n32) * 2 <= nw ? 1 : 0;  // log2 of the parts
+  for (int c = threadIdx.x >> 5; c < (n64 + n32) << split; c += nw) {
+    const bool wide = kPrec && (c >> split) < n64;
+    const int r = (((c >> split) - (wide ? 0 : n64)) << 5) + lane;
+    if (r >= (wide ? count64 : count)) continue;
+    const int e = s.items[wide ? 4 * a.max_slots_pad - 1 - r : r], j = e >> 2, k = e & 3;
+    const int part = c & ((1 << split) - 1);
+    const unsigned parts = split == 0 ? kAllParts : split == 1 ? (part ? 24u : 7u)
+                                                  : (part == 0 ? 8u : part == 1 ? 16u : part == 2 ? 4u : 3u);
     int id[4];
     slot_ids(s.lv[j], id);
     const int idk = k < 2 ? (k == 0 ? id[0] : id[1]) : (k == 2 ? id[2] : id[3]);
@@ -273,13 +229,9 @@ __device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd,
       double g[6];
 #pragma unroll
       for (int q = 0; q < 6; ++q) g[q] = (f >= 0) ? a.coef64[6 * (size_t)f + q] : (double)cf[q * pitch];
-      const float4 r = slot_updates_f64(1u << k, T[0], T[1], T[2], T[3], g[0], g[1], g[2], g[3], g[4], g[5]);
-      u = k < 2 ? (k == 0 ? r.x : r.y) : (k == 2 ? r.z : r.w);
+      u = apex_update64(k, T, g, parts);
     } else {
       const TetGram g = tet_gram9(cf[0], cf[pitch], cf[2 * pitch], cf[3 * pitch], cf[4 * pitch], cf[5 * pitch]);
-      const int part = (c - n64) & ((1 << split) - 1);
-      const unsigned parts = split == 0 ? kAllParts : split == 1 ? (part ? 24u : 7u)
-                                                    : (part == 0 ? 8u : part == 1 ? 16u : part == 2 ? 4u : 3u);
       u = apex_update(k, T, g, parts);
     }
     if (kPhase == 1 && !ownk) {
@@ -321,7 +273,7 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
           need |= (id[k] < nown && m[k] < kLarge3DDev && !plane_skip(T[k], m[k], hs[k]) ? 1u : 0u) << k;
       }
     }
-    append_updates<kPrec>(s, s_n, pm, need, j);
+    append_updates<kPrec>(a, s, s_n, pm, need, j);
   }
   __syncthreads();
   if (tid >= NT - 32) aside();
@@ -378,7 +330,7 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
       s.fl[j] = (unsigned char)(live & ~own);
       s.h0[j] = make_float4(lo[0], lo[1], lo[2], lo[3]);
     }
-    append_updates<kPrec>(s, s_n, pm, need, j);
+    append_updates<kPrec>(a, s, s_n, pm, need, j);
   }
   __syncthreads();
   run_items<0, kPrec>(a, bd, s, s_n, nullptr, pm);
@@ -426,7 +378,7 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
             (unk & 4u) ? ~0u : __float_as_uint(T[2]), (unk & 8u) ? ~0u : __float_as_uint(T[3]));
       }
     }
-    append_updates<kPrec>(s, s_n, pm, need, j);
+    append_updates<kPrec>(a, s, s_n, pm, need, j);
     const unsigned bal = __ballot_sync(0xffffffffu, put);
     if (bal) {
       const unsigned lane = tid & 31u;
@@ -471,7 +423,7 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
           a.fim_memo[bd.slot_begin + j] = make_uint4(__float_as_uint(T[0]), __float_as_uint(T[1]),
                                                      __float_as_uint(T[2]), __float_as_uint(T[3]));
       }
-      append_updates<kPrec>(s, s_n, pm, need, j);
+      append_updates<kPrec>(a, s, s_n, pm, need, j);
     }
     __syncthreads();
     run_items<2, kPrec>(a, bd, s, s_n, nullptr, pm);

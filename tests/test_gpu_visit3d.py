@@ -1,6 +1,6 @@
-"""The 3D item visit (copies put off, one update body for all apexes) against the
-slot-per-thread kernels, which run precision mode with no tet flagged: results, iteration
-and visit counts are equal, bit for bit, over block shapes around a CTA's and a warp's
+"""The 3D item visit (copies put off, one update body for all apexes): the resident loop,
+precision mode with no tet flagged and the kernel-by-kernel loop agree on results,
+iteration and visit counts, bit for bit, over block shapes around a CTA's and a warp's
 size, scalar and anisotropic metrics, slivers, caps and several seeds."""
 import numpy as np
 import pytest
@@ -55,7 +55,7 @@ def _solve(eik, xyz, tets, metric, seeds, vpb, cap, slots, **opts):
     ("cube", 25, 64, 1, [0, 7812, 15000], 2),
     ("cube", 25, 64, 1, [0, 7812, 15000], 7),
 ])
-def test_item_visits_equal_slot_kernels(eik, mg, mesh, n, vpb, metric, seeds, cap):
+def test_item_visits_agree(eik, mg, mesh, n, vpb, metric, seeds, cap):
     xyz, tets = _mesh(mg, mesh, n)
     m = None
     if metric == 1:
