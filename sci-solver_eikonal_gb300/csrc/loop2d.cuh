@@ -22,6 +22,15 @@
 //   * the owned times are kept as two sets of integer keys that swap roles every
 //     sweep, the next set taking the minimum of the candidates, so a sweep has one
 //     CTA barrier and no merge pass;
+//   * where CTAs have several visits an iteration (k_loop2d), one warp fetches the next
+//     visit's descriptor during the sweeps, three dependent reads that began every visit
+//     (a batch of 256 icospheres: 11.8 -> 10.9 ms, 2560 blocks: 1.89 -> 1.80 ms);
+//   * with one lane per slot the slot is turned so that its earliest corner comes last
+//     and its update is nearly always left out (Slot2::turn; the batch: 10.9 -> 10.6 ms).
+//     That batch is bound by latency, not by arithmetic: 8 CTAs an SM wait half of the
+//     time, a fourth of it at the grid barriers.  No gain: ending the sweeps when nothing
+//     changes (0.96x: a reduction in every barrier), one root at a time (0.97x), claims in
+//     place of a fixed order (0.98x), slots fetched ahead into L1 (0.95x);
 //   * the all-vertex test looks only at the vertices that a check wrote (all others
 //     kept their values, which the test would find equal) and at a count of
 //     unreached vertices.
@@ -203,10 +212,39 @@ struct Slot2 {
       if (mine && dead[q])
         dval[q] = a.Tinit[id[q] < bd.nowned ? bd.vbase + id[q] : a.halo[bd.halo_begin + id[q] - bd.nowned]];
   }
+  // One lane per slot, with the block's times staged: turns the slot so that its earliest
+  // corner comes last.  The others' updates then nearly always leave it as it is
+  // (settled2d), and the third update is not run.
+  __device__ __forceinline__ void turn(const Smem2& s, int nown) {
+    float t[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) t[q] = value(s, nown, q);
+    const int by = (t[0] < t[1] && t[0] < t[2]) ? 1 : (t[1] < t[2]) ? 2 : 0;  // new corner q is corner q + by
+    const auto pick = [by](auto& v) {
+      const auto x = v[0], y = v[1], z = v[2];
+      v[0] = by == 0 ? x : by == 1 ? y : z;
+      v[1] = by == 0 ? y : by == 1 ? z : x;
+      v[2] = by == 0 ? z : by == 1 ? x : y;
+    };
+    pick(id);
+    pick(live);
+    pick(dead);
+    pick(dval);
+    pick(e);
+  }
+  // corner q's time at the start of a visit
+  __device__ __forceinline__ float value(const Smem2& s, int nown, int q) const {
+    if (!mine || dead[q]) return dval[q];
+    return id[q] >= nown ? s.halo[id[q] - nown] : __int_as_float(s.key[0][id[q]]);
+  }
+  template <bool kCheck>
+  __device__ __forceinline__ TriConst corner_const(int q) const {
+    return tri_const<kCheck>(e[(q + 1) % 3], e[(q + 2) % 3], e[q], F);
+  }
   template <bool kCheck>
   __device__ __forceinline__ void consts(TriConst* tc) const {
 #pragma unroll
-    for (int q = 0; q < kC; ++q) {
+    for (int q = 0; q < (kLanes == 3 ? 1 : 2); ++q) {
       const int c = corner(q);
       tc[q] = tri_const<kCheck>(c == 0 ? e[1] : c == 1 ? e[2] : e[0], c == 0 ? e[2] : c == 1 ? e[0] : e[1],
                                 c == 0 ? e[0] : c == 1 ? e[1] : e[2], F);
@@ -214,10 +252,17 @@ struct Slot2 {
   }
 };
 
+// Whether no candidate at C (time T) from A and B can be below T: not those along the
+// edges, whose travel times are known, and not one inside, which is a convex combination
+// of TA and TB, off by less than 2^-22 of the larger after rounding, plus a distance.
+__device__ __forceinline__ bool settled2d(float T, float TA, float TB, float EA, float EB) {
+  return T <= __fadd_rn(TA, EA) && T <= __fadd_rn(TB, EB) && T <= __fmaf_rn(fmaxf(TA, TB), -0x1p-20f, fminf(TA, TB));
+}
+
 // n sweeps over the block whose owned times are in both key sets and whose halo times
 // are in s.halo; leaves the final owned times in s.key[n & 1] and those before the last
 // sweep in the other set.  Ends with a CTA barrier (the caller has one before).
-template <int kSweeps, int kLanes>
+template <bool kCheck, int kSweeps, int kLanes>
 __device__ __forceinline__ void sweep2d(const Slot2<kLanes>& sl, const TriConst* tc, const Smem2& s, int nown) {
   constexpr int kC = Slot2<kLanes>::kC;
   const int lane = threadIdx.x & 31;
@@ -259,7 +304,12 @@ __device__ __forceinline__ void sweep2d(const Slot2<kLanes>& sl, const TriConst*
 #pragma unroll
     for (int q = 0; q < kC; ++q) {
       float nw = own[q];
-      if (run) nw = mn2(own[q], tri_candidate(tc[q], TA[q], TB[q]));
+      if (kLanes == 3 || q < 2) {
+        if (run) nw = mn2(own[q], tri_candidate(tc[q], TA[q], TB[q]));
+      } else if (run && !settled2d(own[q], TA[q], TB[q], __fmul_rn(sl.e[q], sl.F), __fmul_rn(sl.e[(q + 2) % 3], sl.F))) {
+        // (see Slot2::turn; its constants are formed here, as they are seldom needed)
+        nw = mn2(own[q], tri_candidate(sl.template corner_const<kCheck>(q), TA[q], TB[q]));
+      }
       // the next set still holds the value before this one (pown): a copy whose value
       // did not fall since then has nothing to add
       if (sl.live[q]) {
@@ -281,8 +331,10 @@ __device__ __forceinline__ void sweep2d(const Slot2<kLanes>& sl, const TriConst*
 }
 
 // Loads block bd with the times of Tsrc and runs kSweeps sweeps on it.
-template <bool kCheck, int kSweeps, int kLanes>
-__device__ __forceinline__ void visit2d(const DevArgs& a, const BlockDesc& bd, const Smem2& s, const float* Tsrc) {
+// `aside` runs in the last warp while the sweeps do: a block's slots seldom reach it.
+template <bool kCheck, int kSweeps, int kLanes, class Aside>
+__device__ __forceinline__ void visit2d(const DevArgs& a, const BlockDesc& bd, const Smem2& s, const float* Tsrc,
+                                        Aside aside) {
   Slot2<kLanes> sl;
   sl.load(a, bd);
   for (int k = threadIdx.x; k < bd.nowned; k += blockDim.x) {
@@ -292,10 +344,15 @@ __device__ __forceinline__ void visit2d(const DevArgs& a, const BlockDesc& bd, c
   }
   for (int k = threadIdx.x; k < bd.nhalo; k += blockDim.x) s.halo[k] = __ldcg(Tsrc + a.halo[bd.halo_begin + k]);
   sl.load_dead(a, bd);
-  TriConst tc[Slot2<kLanes>::kC];
-  sl.template consts<kCheck>(tc);
+  TriConst tc[kLanes == 3 ? 1 : 3];
+  if constexpr (kLanes == 3) sl.template consts<kCheck>(tc);
   __syncthreads();
-  sweep2d<kSweeps, kLanes>(sl, tc, s, bd.nowned);
+  if (threadIdx.x >= blockDim.x - 32) aside();
+  if constexpr (kLanes == 1) {
+    sl.turn(s, bd.nowned);
+    sl.template consts<kCheck>(tc);
+  }
+  sweep2d<kCheck, kSweeps, kLanes>(sl, tc, s, bd.nowned);
 }
 
 // ---------------------------------------------------------------------------
@@ -438,6 +495,32 @@ __global__ void __maxnreg__(kRegs) k_loop2d(DevArgs a, Start2 st) {
   // vertices of the sweeps, then of the checks
   __shared__ unsigned s_cnt[8];
   if (tid < 8) s_cnt[tid] = 0u;
+  // the CTA's present and next item: words 0-7 the block's descriptor, 8 and 9 its range of
+  // neighbours, 10 its instance, 11 the block, 12 whether the instance is finished
+  __shared__ int s_item[2][16];
+  const bool last_warp = tid >= NT - 32;
+  const auto stage = [&](int* to, int b) {  // by one warp
+    int w = 0;
+    if (lane < 8) w = reinterpret_cast<const int*>(a.blocks + b)[lane];
+    else if (lane < 10) w = a.nbr_off[b + lane - 8];
+    else if (lane == 10) w = single ? 0 : a.blk_inst[b];
+    else if (lane == 11) w = b;
+    if (lane < 12) to[lane] = w;
+    if (lane == 10) to[12] = single ? 0 : __ldcg(a.inst_done + w);
+  };
+  const auto item_block = [](const int* d) {
+    BlockDesc bd;
+    bd.slot_begin = d[0];
+    bd.nslots = d[1];
+    bd.nslots_pad = d[2];
+    bd.vbase = d[3];
+    bd.nowned = d[4];
+    bd.halo_begin = d[5];
+    bd.nhalo = d[6];
+    bd.ninside = d[7];
+    return bd;
+  };
+  static_assert(sizeof(BlockDesc) == 32, "staged as eight words");
   while (go) {
     const int stamp = iter + 1;
     const int now = iter % 3, clear = (iter + 1) % 3;
@@ -447,13 +530,24 @@ __global__ void __maxnreg__(kRegs) k_loop2d(DevArgs a, Start2 st) {
     int* const p_next = single ? &y->next[now] : &a.ctl->nnext;
     // ---- sweeps of the active blocks: read Ta, write Tb ----
     if (tid == 0 && blockIdx.x == 0 && st.telemetry && iter < a.ktime_cap) a.ktime[kKStride * iter] = ~global_ns();
-    for (int item = blockIdx.x; item < nact; item += G) {
-      const int b = __ldcg(act + item);
-      const BlockDesc bd = a.blocks[b];
-      const int e0 = a.nbr_off[b], e1 = a.nbr_off[b + 1];
-      if (a.ninst > 1 && __ldcg(a.inst_done + a.blk_inst[b])) continue;  // uniform across the CTA
+    int par = 0;
+    if (last_warp && blockIdx.x < nact) stage(s_item[0], __ldcg(act + blockIdx.x));
+    __syncthreads();
+    for (int item = blockIdx.x; item < nact; item += G, par ^= 1) {
+      const int bn = (last_warp && item + G < nact) ? __ldcg(act + item + G) : -1;
+      const int* const d = s_item[par];
+      const auto ahead = [&] {
+        if (bn >= 0) stage(s_item[par ^ 1], bn);
+      };
+      if (d[12]) {  // uniform across the CTA
+        if (last_warp) ahead();
+        __syncthreads();
+        continue;
+      }
+      const BlockDesc bd = item_block(d);
+      const int e0 = d[8], e1 = d[9];
       const int nb0 = (tid < 32 && e0 + lane < e1) ? a.nbr[e0 + lane] : -1;
-      visit2d<false, 7, kLanes>(a, bd, s, a.Ta);
+      visit2d<false, 7, kLanes>(a, bd, s, a.Ta, ahead);
       int myconv = 1;
       for (int k = tid; k < bd.nowned; k += NT) {
         const float nv = __int_as_float(s.key[1][k]), ov = __int_as_float(s.key[0][k]);
@@ -503,18 +597,31 @@ __global__ void __maxnreg__(kRegs) k_loop2d(DevArgs a, Start2 st) {
     // ---- checks of the active and the queued blocks: read Tb, write Ta ----
     const int count = nact + __ldcg(p_fresh);
     int* nxt = next_list(a, iter);
-    for (int item = blockIdx.x; item < count; item += G) {
-      const int b = (item < nact) ? __ldcg(act + item) : __ldcg(a.list_new + item - nact);
-      const BlockDesc bd = a.blocks[b];
-      const int inst = (a.ninst > 1) ? a.blk_inst[b] : 0;
-      if (a.ninst > 1 && __ldcg(a.inst_done + inst)) continue;
+    const auto queued = [&](int item) { return __ldcg(item < nact ? act + item : a.list_new + item - nact); };
+    par = 0;
+    // (a CTA that had one sweep at most still holds that block's descriptor)
+    if (last_warp && blockIdx.x < count && (blockIdx.x >= nact || nact > G)) stage(s_item[0], queued(blockIdx.x));
+    __syncthreads();
+    for (int item = blockIdx.x; item < count; item += G, par ^= 1) {
+      const int bn = (last_warp && item + G < count) ? queued(item + G) : -1;
+      const int* const d = s_item[par];
+      const auto ahead = [&] {
+        if (bn >= 0) stage(s_item[par ^ 1], bn);
+      };
+      if (d[12]) {
+        if (last_warp) ahead();
+        __syncthreads();
+        continue;
+      }
+      const BlockDesc bd = item_block(d);
+      const int inst = d[10], b = d[11];
       // what the all-vertex test compares with: the times before this check, which are
       // the values it kept, except the caller's initial values in its first iteration
       const float* before =
           (st.user_prev && (a.ninst > 1 ? __ldcg(a.inst_iters + inst) : iter) == 0) ? a.prev : a.Ta;
       const float old0 = (tid < bd.nowned) ? __ldcg(a.Ta + bd.vbase + tid) : 0.0f;
       const float was0 = (before == a.Ta || tid >= bd.nowned) ? old0 : __ldcg(before + bd.vbase + tid);
-      visit2d<true, 1, kLanes>(a, bd, s, a.Tb);
+      visit2d<true, 1, kLanes>(a, bd, s, a.Tb, ahead);
       int myconv = 1, bad = 0, reached = 0;
       for (int k = tid; k < bd.nowned; k += NT) {
         const float nv = __int_as_float(s.key[1][k]), ov = __int_as_float(s.key[0][k]);
@@ -696,7 +803,7 @@ __global__ void __maxnreg__(kRegs) k_blocks2d(DevArgs a, Start2 st) {
       if (tid < bd.nhalo) s.halo[tid] = __ldcg(a.Ta + hid);
       for (int k = tid + NT; k < bd.nhalo; k += NT) s.halo[k] = __ldcg(a.Ta + a.halo[bd.halo_begin + k]);
       __syncthreads();
-      sweep2d<7, kLanes>(sl, tc, s, bd.nowned);
+      sweep2d<false, 7, kLanes>(sl, tc, s, bd.nowned);
       int myconv = 1;
       for (int k = tid; k < bd.nowned; k += NT) {
         const float nv = __int_as_float(s.key[1][k]), ov = __int_as_float(s.key[0][k]);
@@ -727,7 +834,7 @@ __global__ void __maxnreg__(kRegs) k_blocks2d(DevArgs a, Start2 st) {
       for (int k = tid + NT; k < bd.nhalo; k += NT) s.halo[k] = __ldcg(a.Tb + a.halo[bd.halo_begin + k]);
       for (int k = tid; k < bd.nowned; k += NT) s.key[0][k] = s.key[1][k] = __float_as_int(tb[k]);
       __syncthreads();
-      sweep2d<1, kLanes>(sl, tk, s, bd.nowned);
+      sweep2d<true, 1, kLanes>(sl, tk, s, bd.nowned);
       int myconv = 1, bad = 0, reached = 0;
       for (int k = tid; k < bd.nowned; k += NT) {
         const float nv = __int_as_float(s.key[1][k]), ov = __int_as_float(s.key[0][k]);

@@ -24,7 +24,9 @@ def _handle(eik, mg, mesh, n, vpb, seeds, cap=1000, history=0, init=None, speeds
     e.maxVertsPerBlock_ = vpb
     e.maxIterations_ = cap
     e.keepHistory_ = history
-    if speeds:
+    if isinstance(speeds, tuple):
+        e.initSpeedMtxMultipliers((10.0 ** np.random.default_rng(n).uniform(*speeds, len(faces))).astype(np.float32))
+    elif speeds:
         e.initSpeedMtxMultipliers(mg.batch_speed(xyz, faces))
     if init is not None:
         v = np.full(xyz.shape[0], 1e7, np.float32)
@@ -95,6 +97,27 @@ def test_batches_equal_single_solves(eik, mg, levels, vpb):
             h.directLaunch_ = 0
             assert np.array_equal(res[i].view(np.uint32), h.getFinalResult().view(np.uint32)), i
             assert b.numIterations(i) == h.numIterations()
+
+
+def test_batches_of_obtuse_meshes_and_extreme_speeds(eik, mg):
+    """A batch's slots leave out the update of their earliest corner where it cannot fall:
+    equal times, virtual faces, times from 1e-4 to unreachable and the caller's own initial
+    values take every side of that rule."""
+    hs = []
+    for i, (mesh, n, lo, hi) in enumerate([("obtuse", 40, 0, 0), ("grid", 33, 0, 0), ("obtuse", 25, -6, 6),
+                                           ("ico", 3, -30, 30), ("obtuse", 50, -2, 1), ("grid", 9, -37, -36)]):
+        e = _handle(eik, mg, mesh, n, 32, [0, 3 * i + 1], cap=200, init=[5, 6, 11] if i % 2 else None,
+                    speeds=(lo, hi))
+        hs.append(e)
+    b = eik.EikonalBatch(hs)
+    b.solveEikonal()
+    res = [r.copy() for r in b.getFinalResults()]
+    for i, h in enumerate(hs):
+        h.directLaunch_ = 1
+        h.solveEikonal()
+        h.directLaunch_ = 0
+        assert np.array_equal(res[i].view(np.uint32), h.getFinalResult().view(np.uint32)), i
+        assert b.numIterations(i) == h.numIterations()
 
 
 def test_concurrent_solves_of_several_threads(eik, mg):
