@@ -2,12 +2,16 @@
 // the block-partitioned Fast Iterative Method.
 //
 // Reference mapping (paths inside SCI-Solver_Eikonal):
-//   k_sweep3d         FIMCuda           src/core3d/cuda/CUDA_kernels.cu:383-489   (2 sweeps, apex items)
-//   k_check3d         run_check_neghbor CUDA_kernels.cu:493-602                    (1 sweep, flags only)
-//   k_visit3d<false>  FIMCuda, slot per thread (blocks too large for the item kernels'
-//                     shared memory, and precision mode)
+//   k_loop3d          a whole solve of two sweeps a visit (loop3d.cuh)
+//   k_items3d         FIMCuda and run_check_neghbor, src/core3d/cuda/CUDA_kernels.cu:383-602 (2 sweeps and checks, one
+//                     launch an iteration: server, precision mode, kernel-by-kernel loop; visit3d.cuh)
+//   k_sweep3d         FIMCuda and run_check_neghbor, other sweep counts
+//   k_check3d         run_check_neghbor CUDA_kernels.cu:493-602, beside k_visit3d<false>
+//   k_visit3d<false>  FIMCuda, slot per thread (blocks too large for the others' shared
+//                     memory, and the solver without allocations)
 //   k_visit3d<true>   run_check_neghbor, slot per thread (the same cases)
 //   k_commit3d        CopyOutBack + host activation, meshFIM3dEikonal.cu:438-488, CUDA_kernels.cu:604-668
+//   k_loop2d / k_blocks2d  a whole solve or batch of seven sweeps a visit (loop2d.cuh)
 //   k_visit2d_slot / k_visit2d <false>  FIMCuda  src/core2d/cuda/CUDA_kernels.cu:36-409  (7 sweeps)
 //   k_visit2d_slot / k_visit2d <true>   run_check_neighbor CUDA_kernels.cu:415-799    (1 sweep, writes values)
 //   k_activate2d      host activation   src/core2d/cuda/meshFIM2d_eikonal.cu:734-756
@@ -16,9 +20,11 @@
 //   run_reduction (both dims) is a __syncthreads_and inside the visit kernels.
 //
 // Design (GB300-first, not a translation):
-//   * One CTA visits one block at a time: its own index first, then blocks from a
-//     device counter; grids are sized by occupancy x 152 SMs and stay fixed so the
-//     whole iteration is a CUDA-graph body.  A conditional while-node repeats the
+//   * A solve or batch of the reference's sweep counts is one cooperative launch whose
+//     CTAs stay for all iterations and meet at grid barriers.  Elsewhere (server,
+//     precision mode, other sweep counts) one CTA visits one block at a time: its own
+//     index first, then blocks from a device counter; grids are sized by occupancy x 152
+//     SMs and stay fixed so the whole iteration is a CUDA-graph body.  A conditional while-node repeats the
 //     body (four iterations a pass outside the server) until no block is active:
 //     no host round trip per iteration.  Consecutive kernels of the body are joined
 //     by programmatic dependencies.
@@ -158,7 +164,6 @@ struct DevArgs {
   // precision mode's polish: the bounds of the FP64 updates of slots without FP64
   // products, per slot (k_plane_bounds_u64); null: none
   const uint2* hsu64;
-  int sweep_split;  // active blocks from which the large-grid sweep launch runs
   // 3D item path: the neighbour checks of iteration k run inside the sweep kernel
   // of iteration k+1 (they read the same committed times), a block that moves being
   // swept in the same visit.  cand: two lists of nb check candidates (by the parity
@@ -202,16 +207,6 @@ typedef double PrecWide;  // precision mode's wide updates
 // whether the driver accepted programmatic edges in a conditional loop body
 bool g_pdl_ok = true;
 constexpr int kKStride = 16;    // words of per-iteration telemetry (DevArgs::ktime)
-#ifndef EIK_SWEEP_ITEMS
-#define EIK_SWEEP_ITEMS 1
-#endif
-// active blocks below which the 3D sweep runs as 1024-thread CTAs (0: never)
-#ifndef EIK_SWEEP_SPLIT
-#define EIK_SWEEP_SPLIT 0
-#endif
-#ifndef EIK_SWEEP_MEMO
-#define EIK_SWEEP_MEMO 1
-#endif
 // precision mode's polish: every slot's update in FP64 (1) or only the flagged
 // tets' (0), and the relative gap to the FP64 update that re-queues a block
 #ifndef EIK_POLISH_F64ALL
@@ -226,9 +221,6 @@ constexpr int kKStride = 16;    // words of per-iteration telemetry (DevArgs::kt
 #ifndef EIK_ITEM_STEAL
 #define EIK_ITEM_STEAL 1
 #endif
-#ifndef EIK_CHECK_ITEMS
-#define EIK_CHECK_ITEMS 1
-#endif
 // item kernels: CTA size when the caller gives none, and the register cap that
 // lets three such CTAs share an SM's 64 K registers
 #ifndef EIK_ITEM_THREADS
@@ -240,22 +232,11 @@ constexpr int kKStride = 16;    // words of per-iteration telemetry (DevArgs::kt
 #ifndef EIK_PREC_MAXNREG
 #define EIK_PREC_MAXNREG 80
 #endif
-// sweep visits: the block's sweep memos arrive with its bulk copies (1) or are read
-// from memory while the first sweep's updates are listed (0)
-#ifndef EIK_STAGE_SWEEP_MEMO
-#define EIK_STAGE_SWEEP_MEMO 1
-#endif
 #ifndef EIK_SIZED_AUX
 #define EIK_SIZED_AUX 1
 #endif
 #ifndef EIK_TELEMETRY
 #define EIK_TELEMETRY 1
-#endif
-
-// 3D item kernels: the neighbour checks of an iteration run inside the next
-// iteration's sweep launch (1) or as their own launch, k_check3d (0)
-#ifndef EIK_FUSED_CHECK
-#define EIK_FUSED_CHECK 1
 #endif
 
 // ---------------------------------------------------------------------------
@@ -1028,17 +1009,12 @@ __device__ __forceinline__ bool check_pass(const DevArgs& a, const BlockDesc& bd
 }
 
 // at most 56 registers: three CTAs of 384 threads fit one SM's register file
-// role: 0 runs every iteration; where the loop body holds two sweep launches of
-// different CTA sizes, 1 runs only iterations with at least a.sweep_split active
-// blocks and 2 only the others (few blocks: a visit's latency, which more threads
-// per block shorten, sets the launch's time).
 // With a.fused, the CTAs also claim the check candidates queued by the previous
 // iteration's commit (items nact.. of the claim range): a candidate's check runs
 // on the staged block, and a block that moves is appended to this iteration's
 // active list and swept in the same visit.
-__global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a, int role) {
+__global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a) {
   pdl_begin();
-  if (role != 0 && ((a.ctl->nact >= a.sweep_split) != (role == 1))) return;
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int s_item;
@@ -1087,7 +1063,7 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a, int role) {
     SmemItems s = s0;
     // a candidate's check memos, or an active block's sweep memos, arrive in the
     // per-slot copy buffer h0, which the first sweep neither reads nor writes
-    uint4* const smemo = (chk ? a.chk_memo != nullptr : (EIK_STAGE_SWEEP_MEMO && a.fim_memo != nullptr))
+    uint4* const smemo = (chk ? a.chk_memo != nullptr : a.fim_memo != nullptr)
                              ? reinterpret_cast<uint4*>(s.h0)
                              : nullptr;
     if (!load_block(a, bd, 6, s, &bar, parity, a.Ta, smemo, a.hsb ? s.hs : nullptr, chk ? nullptr : a.fim_memo)) {
@@ -2931,16 +2907,8 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
     void* kv_fim;
     void* kv_chk;
     if (L.dim == 3) {
-#if EIK_SWEEP_ITEMS
       kv_fim = P.prec ? (void*)k_visit3d<false, true> : (void*)k_sweep3d;
-#else
-      kv_fim = P.prec ? (void*)k_visit3d<false, true> : (void*)k_visit3d<false>;
-#endif
-#if EIK_CHECK_ITEMS
       kv_chk = P.prec ? (void*)k_visit3d<true, true> : (void*)k_check3d;
-#else
-      kv_chk = P.prec ? (void*)k_visit3d<true, true> : (void*)k_visit3d<true>;
-#endif
       // check visits need one set of per-slot copies; they stage the block's check
       // memos (16 B per slot) behind it, and sweep visits their packed slot list
       // (4 B per slot) behind theirs
@@ -2964,10 +2932,8 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
         CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         const size_t si = smem_bytes_items(P.max_slots_pad, P.max_local, P.max_owned);
         const size_t sc = smem_bytes_check(P.max_slots_pad, P.max_local, P.max_owned);
-#if EIK_SWEEP_ITEMS
         if (!P.prec && si + 64 <= (size_t)maxsm) vsmem = si;
         else if (!P.prec) kv_fim = (void*)k_visit3d<false>;
-#endif
         // the reference's two sweeps have a kernel of their own
         const size_t sv = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, P.prec);
         if (sweeps == 2 && P.chk_memo && sv + 64 <= (size_t)maxsm) {
@@ -2976,18 +2942,12 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
           vsmem = sv;
           a.chk_memo = P.chk_memo;
         }
-#if EIK_SWEEP_MEMO
         if ((kv_fim == (void*)k_sweep3d || items2) && P.chk_memo)
           a.fim_memo = P.chk_memo + P.coef_n / 6;
-#endif
-#if EIK_CHECK_ITEMS
         if (!P.prec && sc + 64 <= (size_t)maxsm) vsmem_chk = sc;
         else if (!P.prec) kv_chk = (void*)k_visit3d<true>;
-#endif
-        (void)si;
-        (void)sc;
       }
-      a.fused = (items2 || (EIK_FUSED_CHECK && kv_fim == (void*)k_sweep3d && kv_chk == (void*)k_check3d)) ? 1 : 0;
+      a.fused = (items2 || (kv_fim == (void*)k_sweep3d && kv_chk == (void*)k_check3d)) ? 1 : 0;
     } else if (slot2d) {
       vthreads = std::max(32, (P.max_slots_pad + 31) & ~31);
       vsmem = vsmem_chk = smem_bytes_slot2d(P.max_slots_pad, P.max_local, P.max_owned);
@@ -3047,9 +3007,9 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
     // consecutive kernels of the body are joined by programmatic edges (every body
     // kernel begins with pdl_begin); where the driver refuses them, ordinary edges
     const bool pdl = EIK_PDL && g_pdl_ok;
-    auto add = [&](void* f, int grid, int block, size_t sm, void** params, int extra = -1) -> std::string {
+    auto add = [&](void* f, int grid, int block, size_t sm, void** params) -> std::string {
       if (record)
-        P.body.push_back(Impl::Launch{f, grid, block, sm, extra >= 0 ? extra : (f == (void*)k_snapshot) ? L.dim : 0});
+        P.body.push_back(Impl::Launch{f, grid, block, sm, (f == (void*)k_snapshot) ? L.dim : 0});
       cudaKernelNodeParams q{};
       q.func = f; q.gridDim = dim3(grid); q.blockDim = dim3(block); q.sharedMemBytes = (unsigned)sm;
       q.kernelParams = params;
@@ -3080,27 +3040,10 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
     static int copy_idx[kBodyCopies] = {0, 1, 2, 3};  // read-only kernel arguments
     static_assert(kBodyCopies == 4, "copy_idx lists every copy");
     const int copies = serve ? 1 : kBodyCopies;
-    // the item sweep at its usual CTA size for iterations with many active blocks
-    // and at 1024 threads for the others (roles of k_sweep3d), each launch leaving
-    // the other's iterations at once
-    static int role_vals[3] = {0, 1, 2};  // read-only kernel arguments
-    void* sweep_args[3][2] = {{&P.args, &role_vals[0]}, {&P.args, &role_vals[1]}, {&P.args, &role_vals[2]}};
-    int grid_small = 0;
-    if (kv_fim == (void*)k_sweep3d && EIK_SWEEP_SPLIT > 0 && vthreads == kItemThreads && !a.fused) {
-      int occ2 = 0;
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_sweep3d, 1024, vsmem));
-      if (occ2 >= 1) grid_small = std::min(occ2 * nsm, std::max(L.nb, 1));
-    }
-    a.sweep_split = grid_small ? EIK_SWEEP_SPLIT : 0;
     for (int u = 0; u < copies; ++u) {
       record = (u == 0);
       void* close_args[] = {&P.args, &copy_idx[u]};
-      if (grid_small) {
-        if (!(e = add(kv_fim, P.grid_visit, vthreads, vsmem, sweep_args[1], 1)).empty()) return e;
-        if (!(e = add(kv_fim, grid_small, 1024, vsmem, sweep_args[2], 2)).empty()) return e;
-      } else if (!(e = add(kv_fim, P.grid_visit, vthreads, vsmem, sweep_args[0], 0)).empty()) {
-        return e;
-      }
+      if (!(e = add(kv_fim, P.grid_visit, vthreads, vsmem, args_ptr)).empty()) return e;
       if (L.dim == 3) {
         if (!(e = add((void*)k_commit3d, grid_blocks, 256, 0, args_ptr)).empty()) return e;
         if (!a.fused && !(e = add(kv_chk, grid_chk, cthreads, vsmem_chk, args_ptr)).empty()) return e;
@@ -3500,27 +3443,21 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   int threads = given ? opt.threads : full_visit_threads(P.max_slots_pad);
   int tune_slot = -1;  // which candidate CTA size this solve measures
   const int tq = P.prec ? 1 : 0;
-  bool items = false;  // the item sweep and check kernels run (their shared memory fits)
-  if (L.dim == 3 && !P.prec && EIK_SWEEP_ITEMS) {
+  // 3D: which kernels' shared memory holds the largest block: the item sweep and check
+  // (items), the visits of the reference's two sweeps (visits)
+  bool items = false, visits = false;
+  if (L.dim == 3) {
     int maxsm = 0, dev = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    items = smem_bytes_items(P.max_slots_pad, P.max_local, P.max_owned) + 64 <= (size_t)maxsm;
+    items = !P.prec && smem_bytes_items(P.max_slots_pad, P.max_local, P.max_owned) + 64 <= (size_t)maxsm;
+    visits = sweeps == 2 && smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, P.prec) + 64 <= (size_t)maxsm;
   }
-  bool items64 = false;  // precision mode's item visits
-  if (L.dim == 3 && P.prec && sweeps == 2) {
-    int maxsm = 0, dev = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    items64 = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, true) + 64 <= (size_t)maxsm;
-  }
-  if (!given && items) {
+  if (!given && (items || visits)) {
     // item kernels: 384-thread CTAs, three per SM where their shared memory allows
     // (65^3 workload: solve 7.85 ms against 7.93 at 512 and 8.4 at one thread per slot)
     threads = kItemThreads;
-  } else if (!given && items64) {
-    threads = kItemThreads;
-  } else if (!given && L.dim == 3) {
+  } else if (!given && L.dim == 3 && !visits) {
     const int full = threads, half = auto_visit_threads(P.max_slots_pad);
     if (half < full) {
       if (P.tune_n[tq] < 3) {  // 0: warm-up, 1: measure 512, 2: measure the full size
@@ -3536,8 +3473,8 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   // 2D solves of the reference's seven sweeps run in one resident kernel (k_loop2d)
   const bool loop2d = L.dim == 2 && sweeps == 7 && !opt.direct_launch && P.max_slots_pad <= 1024;
   // 3D ones of its two sweeps in another (k_loop3d)
-  const bool loop3d = L.dim == 3 && items && sweeps == 2 && !opt.direct_launch;
-  if (!given && (loop3d || items64)) {
+  const bool loop3d = visits && !P.prec && !opt.direct_launch;
+  if (!given && visits && (loop3d || P.prec)) {
     int dev = 0, nsm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
@@ -3907,7 +3844,7 @@ size_t device_footprint(const Layout& L, const Built3D* b) {
   return nb * sizeof(BlockDesc) + ncoef * sizeof(float) + (size_t)L.total_slots * (sizeof(uint2) + sizeof(int)) +
          (L.dim == 3 ? (size_t)L.total_slots * (2 * sizeof(uint4) + sizeof(uint2)) : 0) + nhalo * sizeof(int) +
          ngraph * sizeof(int) +
-         nv * (2 * sizeof(int) + 5 * sizeof(float)) + nb * (9 * sizeof(int) + 1) + 7 * sizeof(int);
+         nv * (2 * sizeof(int) + 5 * sizeof(float)) + nb * ((L.dim == 3 ? 12 : 9) * sizeof(int) + 1) + 7 * sizeof(int);
 }
 
 cudaStream_t new_stream() {
@@ -4011,7 +3948,7 @@ std::string DeviceSolve::serve_setup(const std::vector<ServeSource>& meshes, con
   const bool given = threads == 128 || threads == 256 || threads == 384 || threads == 512 || threads == 768 ||
                      threads == 1024;
   int th = given ? threads : auto_visit_threads(P.max_slots_pad);
-  if (!given && L.dim == 3 && EIK_SWEEP_ITEMS) {
+  if (!given && L.dim == 3) {
     // the item kernels run where their shared memory fits, at the CTA size a
     // plain solve uses
     int dev = 0, maxsm = 0;

@@ -49,6 +49,8 @@ def _solve(eik, xyz, tets, metric, seeds, vpb, cap, slots, **opts):
     ("cube", 17, 64, 0, [2456], 100),
     ("flat", 17, 64, 0, [2456], 100),
     ("cube", 21, 100, 1, [7], 200),
+    ("cube", 21, 280, 1, [7], 200),  # blocks of 2700 and 3000 slots, at the end of what
+    ("cube", 21, 310, 6, [7, 9000], 200),  # shared memory holds
     ("layers", 17, 64, 6, [0, 4000], 300),
     ("layers", 15, 48, 1, [1687], 300),
     ("cube", 25, 64, 6, [0, 7812, 15000], 1),
