@@ -13,8 +13,8 @@ solve (seed -> every block converged).
          L2 is flushed (512 MB write) before every timed solve, outside the events
   e2e    the same metric through the C ABI with host buffers: seeds copied in,
          solve, travel times copied out, wall clock per step
-  roofline  the block-sweep kernel: algorithmic bytes of its launches / their
-         device-timer spans, against the measured HBM copy bandwidth
+  roofline  the loop kernel's visits: algorithmic bytes / the device-timer spans of
+         its iterations, against the measured HBM copy bandwidth
   cpu_baseline  the CPU restatement of the reference scheme (oracle/) with all
          host threads on a bounded sample of the same solve
 
@@ -49,7 +49,7 @@ WORKLOAD = ("plain FIM 3D at scale: 65^3 jittered Kuhn cube (274,625 verts, 1,57
             "log-uniform per-tet speed [0.5, 2] as metric 1/v^2, seed at the centre vertex, 64 verts/block")
 N_GRID = 65
 MAX_ITERS = 100  # the reference default (src/Eikonal.cu:19); the workload converges in 81
-DRAM_PROFILE = "fim3d_items_dram_c3d.txt"  # per-launch DRAM bytes of the sweep and check kernels over one solve
+DRAM_PROFILE = "fim3d_loop_dram_c3d.txt"  # DRAM bytes of the loop kernel's one launch per solve
 
 
 def parse():
@@ -75,7 +75,7 @@ def parse():
     p.add_argument("--no-patterns", action="store_true",
                    help="c3d only: skip the batched / served / precision summaries added to the line")
     p.add_argument("--launch", default="graph", choices=["graph", "direct"],
-                   help="graph: one CUDA-graph launch per solve; direct: kernel by kernel (for ncu)")
+                   help="graph: one launch per solve (precision mode: one CUDA graph); direct: kernel by kernel")
     p.add_argument("--prec-modes", default="fp32,mixed", help="prec: which of fp32 / mixed to run")
     return p.parse_args()
 
@@ -323,7 +323,7 @@ def bench_batch(args, E, torch, world, local):
     plain_ms, plain_upd, plain_wall = [], 0, []
     mismatch = 0
     for k, e in enumerate([] if args.no_plain else solvers):
-        e.solveEikonal()  # upload + graph build
+        e.solveEikonal()  # upload and first solve
         t = time.perf_counter()
         e.solveEikonal()
         r = e.getFinalResult()
@@ -370,11 +370,11 @@ def bench_batch(args, E, torch, world, local):
                 "h2d_bytes_per_step": int(batch.stats()["h2d_bytes"]), "d2h_bytes_per_step": 4 * nv_total},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": None, "peak_source": peak_src,
-                     "kernel": "k_visit2d_slot<false,7> (block sweeps)",
+                     "kernel": "k_loop2d (the sweep phases of its iterations)",
                      "kernel_ms_per_step": fim_ms / args.steps},
         "clocks": clocks,
-        # start + 4 kernels per iteration, the graph body running 4 iterations a pass
-        "gpu_launches": int(sum(1 + 4 * 4 * ((i + 3) // 4) for i in iters)),
+        # one loop kernel per batch
+        "gpu_launches": args.steps,
     }
 
 
@@ -432,17 +432,19 @@ def launch_bytes(its, fused):
     return sweep, check
 
 
-def traffic_vs_algorithmic(its, profile, fused):
+def traffic_vs_algorithmic(its, profile, fused, one_launch):
     """Mean DRAM bytes per launch from the capture beside the mean algorithmic bytes
     of the same launches (same iterations of the same deterministic solve) in this
     run, for the sweep and the check kernel."""
-    rows = launch_dram(profile)
+    rows = launch_dram(profile) if profile else None
     out = {}
     per_launch = launch_bytes(its, fused)
+    if one_launch:  # the loop kernel: its launch runs every iteration
+        per_launch = [[sum(per_launch[0])], [sum(per_launch[1])]]
     for k, (col, name) in enumerate(((0, "sweep"), (1, "check"))):
         alg = per_launch[k]
         if rows:
-            common = [i for i in sorted(rows) if i < len(its) and rows[i][col] > 0]
+            common = [i for i in sorted(rows) if i < len(alg) and rows[i][col] > 0]
             if common:
                 dram = sum(rows[i][col] for i in common) / len(common)
                 a = sum(alg[i] for i in common) / len(common)
@@ -712,7 +714,7 @@ def main():
     e.keepHistory_ = 0
     e.directLaunch_ = 1 if args.launch == "direct" else 0
     t0 = time.perf_counter()
-    e.solveEikonal()  # partition, layout built on the device, graph build, first solve
+    e.solveEikonal()  # partition, layout built on the device, first solve
     setup_s = time.perf_counter() - t0
     # the same first solve with the block layout built on the host
     eh = E.Eikonal(False)
@@ -737,9 +739,9 @@ def main():
             torch.distributed.barrier()
         torch.cuda.synchronize()
 
-    # the timed solves record no per-launch telemetry (it costs about 1.5%); the same
-    # solve with it, right after, gives the sweep kernel's launch spans and each
-    # launch's visit counts (same bits, same launches) for the roofline
+    # the timed solves record no per-iteration telemetry (it costs about 1.5%); the same
+    # solve with it, right after, gives the iterations' spans and visit counts (same
+    # bits) for the roofline
     e.telemetry_ = 0
     for _ in range(args.warmup):
         e.solveEikonal()
@@ -768,14 +770,14 @@ def main():
     e.solveEikonal()
     st = e.stats()
     its = e.iterationStats()
-    # the checks run inside the sweep kernel: no check launches, check visits counted
+    # the checks run in the sweeps' phase: no check phases, check visits counted
     fused = st["check_launches"] == 0 and st["check_visits"] > 0
     fim_ms, chk_ms = st["fim_kernel_ms"] * args.steps, st["check_kernel_ms"] * args.steps
     fim_bytes = sum(launch_bytes(its, fused)[0]) * args.steps
-    # the state initialisation (k_init_state, k_seed_state), the graph's start node,
-    # then 3 kernels (sweep with checks, commit, close) or 4 per iteration, the graph
-    # body running 4 iterations a pass (loop iterations = sweep launches)
-    launches = args.steps * (3 + (3 if fused else 4) * 4 * ((st["fim_launches"] + 3) // 4))
+    # one k_loop3d per solve; kernel by kernel the state initialisation (k_init_state,
+    # k_seed_state), then 3 kernels (sweep with checks, commit, close) or 4 per iteration
+    one_launch = args.launch == "graph"
+    launches = args.steps * (1 if one_launch else 2 + (3 if fused else 4) * st["fim_launches"])
     e.telemetry_ = 0
     total_ms, upd_all = aggregate_replicas(torch, sum(times), upd, world, "cuda")
     value = upd_all / (total_ms * 1e-3)
@@ -810,7 +812,7 @@ def main():
     else:
         peak, peak_src = 6800.0, "fallback"
     achieved = fim_bytes / (fim_ms * 1e-3) / 1e9 if fim_ms > 0 else 0.0
-    tva = traffic_vs_algorithmic(its, DRAM_PROFILE, fused)
+    tva = traffic_vs_algorithmic(its, DRAM_PROFILE if one_launch else None, fused, one_launch)
     lat = sorted(times)
     res = {
         "metric": METRIC, "value": value, "unit": "vertex-updates/s", "n_gpus": world, "steps": args.steps,
@@ -824,30 +826,30 @@ def main():
         "setup_s": setup_s,
         "first_solve_s": {"device_setup": setup_s, "host_setup": setup_host_s,
                           "bitwise_equal": same_as_host,
-                          "note": "first solve of this mesh (partition, layout, upload, graph, solve) in a "
+                          "note": "first solve of this mesh (partition, layout, upload, solve) in a "
                                   "process whose kernels are loaded"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": tva["sweep"]["traffic"], "peak_source": peak_src,
-                     "kernel": ("k_sweep3d (block sweeps and the previous iteration's neighbour checks)"
-                                if fused else "k_sweep3d (block sweeps)"),
+                     "kernel": ("k_loop3d (all iterations of a solve: block sweeps and the previous iteration's "
+                                "neighbour checks)" if one_launch else "k_items3d (block sweeps and checks)"),
                      "kernel_ms_per_step": fim_ms / args.steps,
-                     "kernel_ms_source": "device-timer span of every sweep launch of one solve with telemetry "
-                                         "on, run right after the timed solves (same launches and bits)",
+                     "kernel_ms_source": "device-timer spans of the iterations' visits in one solve with telemetry "
+                                         "on, run right after the timed solves (same launch and bits)",
                      "algorithmic_bytes_per_launch": tva["sweep"]["algorithmic"],
                      "traffic_over_algorithmic": tva["sweep"]["traffic_over_algorithmic"],
                      "check_kernel": (None if fused else dict(tva["check"], kernel_ms_per_step=chk_ms / args.steps)),
                      "traffic_source": f"profiles/{DRAM_PROFILE}: ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                                       "of every sweep launch of one solve of this workload (kernel by kernel; cold "
-                                       "caches), set beside this run's algorithmic bytes of the same launches",
-                     "note": "the sweep kernel is bound by CTA barriers and instruction latency in the tet local "
-                             "solver, not by HBM",
-                     # compute side, from the committed full capture of one sweep launch (outer
-                     # iteration 40 of the same solve, kernel-by-kernel mode)
-                     "compute": {"bound": "issue", "issue_active_pct": 50.5, "ipc_per_sm": 2.05,
-                                 "fma_pipe_pct": 16.0, "alu_pipe_pct": 30.9, "xu_pipe_pct": 7.3,
+                                       "of the one launch of a solve of this workload (cold caches at its start; "
+                                       "L2 serves the later visits), set beside this run's algorithmic bytes of the "
+                                       "same launch",
+                     "note": "the loop kernel is bound by CTA and grid barriers and by instruction latency in the "
+                             "tet local solver, not by HBM",
+                     # compute side, from the committed capture of one solve's launch
+                     "compute": {"bound": "latency", "issue_active_pct": 34.1, "ipc_per_sm": 1.35,
+                                 "fma_pipe_pct": 9.9, "alu_pipe_pct": 22.4, "xu_pipe_pct": 4.3,
                                  "top_stall": "barrier",
-                                 "source": "ncu --set full capture of one k_sweep3d launch (outer iteration 40) "
-                                           "of this workload, summarised under profiles/"}},
+                                 "source": "ncu capture of one k_loop3d launch of this workload, summarised in "
+                                           "profiles/fim_loops.md"}},
         "e2e": {"value": e2e_value, "unit": "vertex-updates/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": 1e3 * statistics.median(e2e_times),
                 "note": "each step re-solves the resident mesh through the C ABI: seeds copied in, the solve, the "
@@ -1009,7 +1011,7 @@ def first_solve_2d(E, batch_count=256, vpb=128):
     a, h = res["device_setup"], res["host_setup"]
     out["bitwise_equal"] = bool(np.array_equal(a[0].view(np.uint32), h[0].view(np.uint32)) and all(
         np.array_equal(x.view(np.uint32), y.view(np.uint32)) for x, y in zip(a[1], h[1])))
-    out["note"] = ("first solve = partition, block layout, upload, graph and solve (results copied back); "
+    out["note"] = ("first solve = partition, block layout, upload and solve (results copied back); "
                    "the triangle preparation is host work in both builds")
     return out
 
