@@ -1243,8 +1243,8 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a) {
 
 // ===========================================================================
 // 3D sweeps and checks of one iteration (the reference's two sweeps; k_sweep3d runs
-// other sweep counts).  CTAs claim the active blocks, then the check candidates queued
-// by the previous iteration's commit; a candidate that moves is appended to this
+// other sweep counts).  CTAs claim the check candidates queued by the previous
+// iteration's commit, then the active blocks; a candidate that moves is appended to this
 // iteration's active list and swept in the same visit.
 // ===========================================================================
 template <bool kPrec>
@@ -1263,9 +1263,7 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
   const int nact = ctl->nact;
   const int* cand = a.cand + (size_t)((iter + 1) & 1) * a.nb;
   const int ncand = ctl->ncand[(iter + 1) & 1], count = nact + ncand;
-  // with more active blocks than CTAs the candidates come first, so that the sweeps, all
-  // alike, end the launch (see k_loop3d)
-  const bool early = nact > (int)gridDim.x;
+  // the candidates come first, so that the sweeps, all alike, end the launch (see k_loop3d)
   int* list = act_list(a, iter);
   const PrecMode pm = kPrec ? PrecMode{ctl->f64_all, ctl->polish} : PrecMode{0, 0};
   stamp_start(a, iter, 0);
@@ -1280,8 +1278,8 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
   // spares every visit the instance lookup
   const int done1 = (a.ninst == 1) ? a.inst_done[0] : -1;
   while (item < count) {
-    const bool chk = early ? item < ncand : item >= nact;  // a check candidate
-    const int b = early ? (chk ? cand[item] : list[item - ncand]) : (chk ? cand[item - nact] : list[item]);
+    const bool chk = item < ncand;  // a check candidate
+    const int b = chk ? cand[item] : list[item - ncand];
     const BlockDesc bd = a.blocks[b];
     // instance finished: leave its blocks alone; at its cap: its checks only
     const int ist = done1 >= 0 ? done1 : a.inst_done[a.blk_inst[b]];
@@ -1299,7 +1297,7 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
           __syncthreads();
         }
         if (chk) {
-          const bool moved = check_visit3d<kPrec>(a, bd, s, s_n, &s_moved, [] {}, pm);
+          const bool moved = check_visit3d<kPrec>(a, bd, s, s_n, &s_moved, pm);
           if (tid == 0) {  // the previous iteration's check (run_check_neghbor)
             atomicAdd(&ctl->chk_visits, 1ull);
             atomicAdd(&ctl->updates, (unsigned long long)nown);
@@ -1312,7 +1310,7 @@ __global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items
           sweep = sweep && moved;
         }
         if (sweep) {
-          sweep_visit3d<kPrec>(a, bd, s, s_n, chk, true, [] {}, pm);
+          sweep_visit3d<kPrec>(a, bd, s, s_n, chk, true, pm);
           int myconv = 1;
           for (int k = tid; k < nown; k += NT) {
             const float ov = __int_as_float(s.v1[k]), nv = __int_as_float(s.v2[k]);

@@ -112,23 +112,21 @@ struct Loop3 {
   int snap;                 // history row of the last pass's times, or -1
   int state;                // a single solve's: 0 running, 2 at its cap with checks left
   int go;
-  int early;                // this pass's candidates come first
 };
 
-// A pass ends when its last visits do, so its order matters: a sweep takes about 30,000
-// cycles, a check 6,000, and one check in five goes on to a sweep.  With more active
-// blocks than CTAs the candidates come first and the sweeps, all alike, end the pass (97^3
-// cube: the mean wait at the barrier fell from 50,000 cycles to under 30,000, solve 8.30 ->
-// 7.76 ms; 65^3 3.53 -> 3.28 ms); with fewer, the checks fill the CTAs that the sweeps
-// leave.  Claiming the next item during a visit hides its chain of four loads, but the
-// item then waits for this CTA: only while two more rounds of items are left (kAhead).
-constexpr int kAhead = 2;
+// A pass ends when its last visits do, so its order matters: a sweep takes about 25,000
+// cycles, a check 7,000, and one check in five goes on to a sweep.  So the check candidates
+// come first, the sweeps, all alike, fill the CTAs that they leave, and an item is claimed
+// only when its CTA is free.  (65^3 cube: mean visits per CTA and pass 37,000 cycles, mean
+// wait at the barrier 37,700 with the sweeps first while they are fewer than the CTAs and
+// the next item claimed during a visit, which hides its chain of four loads but holds it;
+// solve 3.14 -> 2.87 ms, 41^3 1.82 -> 1.71, 97^3 7.53 -> 7.43.)
 
 // One item of a pass: a block, whether it is a check candidate (flags 1), which of its
 // memos are this solve's (2 check, 4 sweep), whether its instance does not run (16), and
 // if so whether it is at its cap (32: its checks still run).
 struct Item3 {
-  int b, flags, index;
+  int b, flags;
   BlockDesc bd;
 };
 // The CTA's next item (b = -1: none), by one thread: the CTA's index first, then from the
@@ -136,18 +134,16 @@ struct Item3 {
 // (and may have been swept from there in this one by now): passed over.
 __device__ __forceinline__ void next_item(const DevArgs& a, const Start3& st, const volatile Loop3& v, bool first,
                                           volatile Item3& o) {
-  const int iter = v.iter, nact = v.nact, count = nact + v.ncand, G = (int)gridDim.x;
+  const int iter = v.iter, count = v.nact + v.ncand, G = (int)gridDim.x;
   for (;; first = false) {
     const int i = first ? (int)blockIdx.x : count <= G ? count : G + atomicAdd(&st.turn[iter % 3].work, 1);
     if (i >= count) {
       o.b = -1;
       return;
     }
-    const bool early = v.early != 0;
-    const bool chk = early ? i < v.ncand : i >= nact;
-    const int* cand = a.cand + (size_t)((iter + 1) & 1) * a.nb;
-    const int b = __ldcg(early ? (chk ? cand + i : act_list(a, iter) + i - v.ncand)
-                               : (chk ? cand + i - nact : act_list(a, iter) + i));
+    const int ncand = v.ncand;
+    const bool chk = i < ncand;
+    const int b = __ldcg(chk ? a.cand + (size_t)((iter + 1) & 1) * a.nb + i : act_list(a, iter) + i - ncand);
     const BlockDesc bd = a.blocks[b];
     const int sa = __ldcg(a.stampA + b), valid = __ldcg(st.mvalid + b);
     const int ist = a.ninst == 1 ? v.state : __ldcg(a.inst_done + a.blk_inst[b]);
@@ -160,7 +156,6 @@ __device__ __forceinline__ void next_item(const DevArgs& a, const Start3& st, co
     o.bd.nowned = bd.nowned;
     o.bd.halo_begin = bd.halo_begin;
     o.bd.nhalo = bd.nhalo;
-    o.index = i;
     o.b = b;
     return;
   }
@@ -237,7 +232,6 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
     v.iter = v.iters = v.ncand = v.nconv = v.state = 0;
     v.nact = st.nact;
     v.snap = -1;
-    v.early = 0;
     v.go = st.nact > 0 && a.ctl->max_iters > 0;
   }
   __syncthreads();
@@ -252,13 +246,6 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
     __syncthreads();
     for (int cur = 0; s_it[cur].b >= 0; cur ^= 1) {
       const volatile Item3& it = s_it[cur];
-      bool ahead = false;  // (the last warp's first thread) the next item stands ready
-      auto aside = [&] {
-        if (tid == NT - 32 && !ahead && it.index + kAhead * G < v.nact + v.ncand) {
-          next_item(a, st, v, false, s_it[cur ^ 1]);
-          ahead = true;
-        }
-      };
       const bool chk = (it.flags & 1) != 0, run = (it.flags & 16) == 0;  // run: the instance runs
       bool sweep = false, kept = !run && !(chk && (it.flags & 32));
       if (!kept) {
@@ -281,13 +268,13 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
           __syncthreads();
           sweep = run;
           if (chk) {
-            const bool moved = check_visit3d(a, bd, s, s_n, &s_moved, aside);
+            const bool moved = check_visit3d(a, bd, s, s_n, &s_moved);
             sweep = sweep && moved;
             if (tid == 0 && !moved) st.mvalid[it.b] = ((it.flags >> 1) & 3) | 1;
             if (!sweep)  // its times stand in the next buffer too
               for (int k = tid; k < it.bd.nowned; k += NT) buf_out(a, v.iter)[it.bd.vbase + k] = s.vt[k];
           }
-          if (sweep) sweep_visit3d(a, bd, s, s_n, chk, (it.flags & 4) != 0, aside);
+          if (sweep) sweep_visit3d(a, bd, s, s_n, chk, (it.flags & 4) != 0);
         }
         if (chk && tid == 0) {
           s_cnt[4] += 1u;
@@ -366,7 +353,7 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
           }
         }
       }
-      if (tid == NT - 32 && !ahead) next_item(a, st, v, false, s_it[cur ^ 1]);
+      if (tid == NT - 32) next_item(a, st, v, false, s_it[cur ^ 1]);
       __syncthreads();
     }
     copy_settled(a, st.conv + (size_t)((v.iter + 1) & 1) * a.nb, v.nconv, st.queued[(v.iter + 1) & 1], v.iter,
@@ -403,7 +390,6 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
       }
       v.nact = nn;
       v.ncand = nc;
-      v.early = nn > G;
       v.iter = iter + 1;
       if (gtid == 0 && a.ktime && iter < a.ktime_cap) a.ktime[kKStride * iter + 1] = global_ns();
     }

@@ -247,10 +247,9 @@ __device__ __forceinline__ void run_items(const DevArgs& a, const BlockDesc& bd,
 
 // One check of a loaded block (its check memos in h0): whether it moves.  s_n: two
 // counters, zero on entry and on return.  All threads; ends behind a CTA barrier.
-// `aside` runs in the CTA's last warp while the others update: the items seldom reach it.
-template <bool kPrec = false, class Aside>
+template <bool kPrec = false>
 __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, int* s_n,
-                                              volatile int* s_moved, Aside aside, PrecMode pm = PrecMode{0, 0}) {
+                                              volatile int* s_moved, PrecMode pm = PrecMode{0, 0}) {
   const int tid = threadIdx.x, NT = blockDim.x, ns = bd.nslots, nown = bd.nowned;
   if (tid == 0) *s_moved = 0;
   for (int j0 = 0; j0 < ns; j0 += NT) {
@@ -276,7 +275,6 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
     append_updates<kPrec>(a, s, s_n, pm, need, j);
   }
   __syncthreads();
-  if (tid >= NT - 32) aside();
   run_items<0, kPrec>(a, bd, s, s_n, s_moved, pm);
   __syncthreads();
   const bool moved = *s_moved != 0;
@@ -296,9 +294,9 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
 // The two sweeps of a loaded block (its sweep memos in h0, or behind a check read from
 // memory, where `memo` says they are of this solve): the final owned times in v2, those after the first sweep in v1.  s_n as above.
 // Ends behind a CTA barrier.
-template <bool kPrec = false, class Aside>
+template <bool kPrec = false>
 __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, int* s_n,
-                                              bool checked, bool memo, Aside aside, PrecMode pm = PrecMode{0, 0}) {
+                                              bool checked, bool memo, PrecMode pm = PrecMode{0, 0}) {
   const int tid = threadIdx.x, NT = blockDim.x, ns = bd.nslots, nown = bd.nowned;
   // ---- first sweep: owned apexes; bounds of the copies ----
   for (int j0 = 0; j0 < ns; j0 += NT) {
@@ -389,7 +387,6 @@ __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc&
     }
   }
   __syncthreads();
-  if (tid >= NT - 32) aside();
   run_items<1, kPrec>(a, bd, s, s_n, nullptr, pm);
   __syncthreads();
   const int nd = s_n[1];
