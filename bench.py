@@ -845,8 +845,8 @@ def main():
                      "note": "the loop kernel is bound by CTA and grid barriers and by instruction latency in the "
                              "tet local solver, not by HBM",
                      # compute side, from the committed capture of one solve's launch
-                     "compute": {"bound": "latency", "issue_active_pct": 34.1, "ipc_per_sm": 1.35,
-                                 "fma_pipe_pct": 9.9, "alu_pipe_pct": 22.4, "xu_pipe_pct": 4.3,
+                     "compute": {"bound": "latency", "issue_active_pct": 37.1, "ipc_per_sm": 1.47,
+                                 "fma_pipe_pct": 11.1, "alu_pipe_pct": 24.7, "xu_pipe_pct": 4.8,
                                  "top_stall": "barrier",
                                  "source": "ncu capture of one k_loop3d launch of this workload, summarised in "
                                            "profiles/fim_loops.md"}},

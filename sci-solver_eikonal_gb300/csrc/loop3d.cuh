@@ -3,7 +3,7 @@
 //
 // k_loop3d runs a whole 3D solve or batch with the visits of visit3d.cuh.  As three
 // kernels of a CUDA graph per iteration (visits, commit, close; 17^3 cube 775 us, 41^3
-// 2.06 ms, 65^3 3.43 ms, 97^3 7.90 ms a solve, against 597 us, 1.89, 3.28 and 7.76 ms) an
+// 2.06 ms, 65^3 3.43 ms, 97^3 7.90 ms a solve, against 470 us, 1.68, 2.80 and 7.28 ms) an
 // iteration spent 7-8 us between its visits' end and the next one's first loads, a quarter
 // of it where a few dozen blocks are active.  Here an iteration has one grid barrier and no commit
 // step:
