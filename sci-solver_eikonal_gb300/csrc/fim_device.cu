@@ -2480,9 +2480,9 @@ constexpr int kItemThreads = EIK_ITEM_THREADS;
 // gives none.  A mesh's blocks are active a fraction at a time: while fewer are than the
 // GPU holds CTAs, more warps per visit shorten it; when they fill the GPU, three visits
 // per SM overlap better.  Solves on one GB300 in us at 384 / 512 / 768 threads (three, two
-// and one CTA per SM): 562 blocks 1088 / 969 / 948, 792 blocks 1338 / 1238 / 1188, 1077
-// blocks 1482 / 1392 / 1414, 2894 blocks 2826 / 2733 / 3121, 4292 blocks 3156 / 3186 /
-// 4014.
+// and one CTA per SM): 562 blocks 1016 / 917 / 869, 792 blocks 1252 / 1117 / 1111, 1077
+// blocks 1423 / 1303 / 1359, 1839 blocks 1870 / 1812 / 2088, 2894 blocks 2325 / 2337 / 2885,
+// 4292 blocks 2776 / 2888 / 3763.
 int items_threads(int nb, int nsm, bool prec) {
   if (nb <= 6 * nsm) return 768;
   return (nb <= 24 * nsm && !prec) ? 512 : kItemThreads;

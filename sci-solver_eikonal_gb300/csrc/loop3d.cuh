@@ -120,7 +120,7 @@ struct Loop3 {
 // only when its CTA is free.  (65^3 cube: mean visits per CTA and pass 37,000 cycles, mean
 // wait at the barrier 37,700 with the sweeps first while they are fewer than the CTAs and
 // the next item claimed during a visit, which hides its chain of four loads but holds it;
-// solve 3.14 -> 2.87 ms, 41^3 1.82 -> 1.71, 97^3 7.53 -> 7.43.)
+// solve 3.14 -> 2.80 ms, 41^3 1.82 -> 1.68, 97^3 7.53 -> 7.28.)
 
 // One item of a pass: a block, whether it is a check candidate (flags 1), which of its
 // memos are this solve's (2 check, 4 sweep), whether its instance does not run (16), and
