@@ -2746,10 +2746,9 @@ void DeviceSolve::Impl::fill_args(DevArgs& a, const Layout& L, int sweeps, int h
 //     thread), up to five CTAs an SM: 640 blocks took 12.3 us an iteration against
 //     16.0 with lists, 1,849 blocks 3.4 times the lists' time (every CTA meets at every
 //     barrier, most of them with nothing to do).
-//   * Else the active list (k_loop2d).  One solve: a few hundred active blocks, latency
-//     counts, three lanes per slot.  A batch: thousands of active blocks, throughput
-//     counts, one lane per slot (256 icospheres at 32 vertices per block 9.8 ms against
-//     12.5 with three lanes, which load every slot three times).
+//   * Else the active list (k_loop2d), with three lanes per slot or one (below; 256
+//     icospheres at 32 vertices per block 9.8 ms against 12.5 with three lanes, which load
+//     every slot three times).
 // Three lanes need blocks of at most 320 slots (1024 threads).
 std::string DeviceSolve::Impl::choose_loop2d(const Layout& L) {
   Impl& P = *this;
@@ -2770,12 +2769,25 @@ std::string DeviceSolve::Impl::choose_loop2d(const Layout& L) {
       P.loop_grid = L.nb;
       return "";
     }
-  const bool three = L.ninst <= 1 && threads[0] <= 1024;
-  const void* f = three ? (const void*)k_loop2d<3, 64> : (const void*)k_loop2d<1, 64>;
-  P.loop_threads = threads[three ? 0 : 1];
+  // Three lanes per slot shorten a visit, one fills the GPU better.  A single solve's front
+  // is few blocks at a time.  A batch's is a share of its blocks: up to nine of them per
+  // CTA, three lanes are the faster (us per batch at 4, 6, 7 and 9 blocks per three-lane
+  // CTA: 553 against 612, 576 against 627, 946 against 1077, 747 against 782; at 12: 1162
+  // against 1164 and 1168 against 1022, at 32: 2029 against 1873).
   P.loop_smem = smem_bytes_loop2d(P.max_local, P.max_owned, false);
-  CK(raise_smem_limit(f, P.loop_smem));
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, P.loop_threads, P.loop_smem));
+  const void* f = (const void*)k_loop2d<3, 64>;
+  bool three = threads[0] <= 1024;
+  if (three) {
+    CK(raise_smem_limit(f, P.loop_smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads[0], P.loop_smem));
+    three = occ >= 1 && (L.ninst <= 1 || L.nb <= 9ll * occ * nsm);
+  }
+  P.loop_threads = threads[three ? 0 : 1];
+  if (!three) {
+    f = (const void*)k_loop2d<1, 64>;
+    CK(raise_smem_limit(f, P.loop_smem));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, P.loop_threads, P.loop_smem));
+  }
   if (occ < 1) return "loop kernel cannot be resident (shared memory / registers)";
   P.loop_func = f;
   P.loop_grid = std::max(1, std::min(occ * nsm, L.nb));

@@ -99,18 +99,21 @@ def test_batches_equal_single_solves(eik, mg, levels, vpb):
             assert b.numIterations(i) == h.numIterations()
 
 
-def test_batches_of_obtuse_meshes_and_extreme_speeds(eik, mg):
-    """A batch's slots leave out the update of their earliest corner where it cannot fall:
-    equal times, virtual faces, times from 1e-4 to unreachable and the caller's own initial
-    values take every side of that rule."""
+# resident blocks, lists with three lanes, lists with one lane per slot
+@pytest.mark.parametrize("grow,blocks", [(1, (1, 760)), (2.5, (761, 2736)), (4.5, (2737, 20000))])
+def test_batches_of_obtuse_meshes_and_extreme_speeds(eik, mg, grow, blocks):
+    """With one lane per slot a batch leaves out the update of a slot's earliest corner
+    where it cannot fall: equal times, virtual faces, times from 1e-4 to unreachable and the
+    caller's own initial values take every side of that rule."""
     hs = []
     for i, (mesh, n, lo, hi) in enumerate([("obtuse", 40, 0, 0), ("grid", 33, 0, 0), ("obtuse", 25, -6, 6),
                                            ("ico", 3, -30, 30), ("obtuse", 50, -2, 1), ("grid", 9, -37, -36)]):
-        e = _handle(eik, mg, mesh, n, 32, [0, 3 * i + 1], cap=200, init=[5, 6, 11] if i % 2 else None,
-                    speeds=(lo, hi))
+        e = _handle(eik, mg, mesh, int(n * grow) if mesh != "ico" else n, 32, [0, 3 * i + 1], cap=200,
+                    init=[5, 6, 11] if i % 2 else None, speeds=(lo, hi))
         hs.append(e)
     b = eik.EikonalBatch(hs)
     b.solveEikonal()
+    assert blocks[0] <= b.stats()["num_blocks"] <= blocks[1]
     res = [r.copy() for r in b.getFinalResults()]
     for i, h in enumerate(hs):
         h.directLaunch_ = 1
