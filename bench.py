@@ -848,8 +848,8 @@ def main():
                      "compute": {"bound": "latency", "issue_active_pct": 37.1, "ipc_per_sm": 1.47,
                                  "fma_pipe_pct": 11.1, "alu_pipe_pct": 24.7, "xu_pipe_pct": 4.8,
                                  "top_stall": "barrier",
-                                 "source": "ncu capture of one k_loop3d launch of this workload, summarised in "
-                                           "profiles/fim_loops.md"}},
+                                 "source": "ncu capture of one k_loop3d launch of this workload, summarised "
+                                           "under profiles/"}},
         "e2e": {"value": e2e_value, "unit": "vertex-updates/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h, "ms_per_step": 1e3 * statistics.median(e2e_times),
                 "note": "each step re-solves the resident mesh through the C ABI: seeds copied in, the solve, the "
