@@ -2473,6 +2473,18 @@ cudaError_t raise_smem_limit(const void* func, size_t bytes) {
   return cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
+// Whether a CTA of a kernel with `dynamic` bytes of dynamic shared memory can be given
+// them: what the kernel declares itself counts against the same limit.
+std::string fits_shared(const void* func, size_t dynamic, bool* fits) {
+  int dev = 0, maxsm = 0;
+  cudaFuncAttributes fa{};
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CK(cudaFuncGetAttributes(&fa, func));
+  *fits = dynamic + fa.sharedSizeBytes <= (size_t)maxsm;
+  return "";
+}
+
 // CTA size of the item sweep and check kernels when the caller gives none
 constexpr int kItemThreads = EIK_ITEM_THREADS;
 
@@ -2638,7 +2650,7 @@ struct DeviceSolve::Impl {
   }
   size_t smem = 0;
   int grid_visit = 0, grid_aux = 0;
-  const void* loop_func = nullptr;  // 2D loop kernel of the layout and its launch shape, chosen at its first solve
+  const void* loop_func = nullptr;  // loop kernel of the layout and its launch shape, chosen at its first solve
   int loop_grid = 0, loop_threads = 0;
   size_t loop_smem = 0;
   void* opt_stream = nullptr;  // the solver's stream
@@ -2692,9 +2704,9 @@ struct DeviceSolve::Impl {
   void fill_args(DevArgs& a, const Layout& L, int sweeps, int hcap, bool serve, bool tele) const;
   std::string build_graph(const Layout& L, int sweeps, int threads, int hcap, bool serve);
   std::string choose_loop2d(const Layout& L);
+  std::string choose_loop3d(const Layout& L, int threads, bool* resident);
   std::string stage_inputs(size_t o_words, const std::vector<int>& cap, int max_iters, int** words);
-  std::string run_loop3d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap,
-                         int threads);
+  std::string run_loop3d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap);
   std::string run_loop2d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap);
   void drop_graph() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -2822,9 +2834,38 @@ std::string DeviceSolve::Impl::run_loop2d(const Layout& L, const SolveOptions& o
   return "";
 }
 
-// One 3D solve or batch in k_loop3d, enqueued on the solver's stream.
+// The 3D loop kernel of a layout and its launch shape at a CTA size; *resident: whether the
+// GPU holds a CTA of it.  (It keeps 200 bytes of its own where k_items3d keeps 32: blocks
+// of 3364 slots, 460 owned and 801 local vertices fit the one and not the other.)
+std::string DeviceSolve::Impl::choose_loop3d(const Layout& L, int threads, bool* resident) {
+  Impl& P = *this;
+  if (!P.loop_func || P.loop_threads != threads) {
+    int dev = 0, nsm = 0, occ = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    const size_t smem = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, false);
+    // as many registers as the CTAs that shared memory lets an SM hold leave
+    const void* f = threads <= 384 ? (const void*)k_loop3d<56> : threads <= 512 ? (const void*)k_loop3d<64>
+                    : threads <= 768 ? (const void*)k_loop3d<80> : (const void*)k_loop3d<64>;
+    bool fits = false;
+    std::string e = fits_shared(f, smem, &fits);
+    if (!e.empty()) return e;
+    if (fits) {
+      CK(raise_smem_limit(f, smem));
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads, smem));
+    }
+    P.loop_func = f;
+    P.loop_threads = threads;
+    P.loop_smem = smem;
+    P.loop_grid = std::min(occ * nsm, std::max(L.nb, 1));
+  }
+  *resident = P.loop_grid > 0;
+  return "";
+}
+
+// One 3D solve or batch in k_loop3d (choose_loop3d), enqueued on the solver's stream.
 std::string DeviceSolve::Impl::run_loop3d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap,
-                                          int max_iters, int hcap, int threads) {
+                                          int max_iters, int hcap) {
   Impl& P = *this;
   cudaStream_t st = (cudaStream_t)opt_stream;
   std::string e;
@@ -2847,24 +2888,9 @@ std::string DeviceSolve::Impl::run_loop3d(const Layout& L, const SolveOptions& o
   Start3 s3{w, w + ni, w + 2 * ni, w + 2 * ni + nseed, (int)nseed, (int)nact,
             reinterpret_cast<Turn3*>(P.stage + o_turn), reinterpret_cast<GridFlag*>(P.stage + o_flags),
             P.loop3_lists, P.loop3_lists + 2 * (size_t)L.nb, {P.stampC, P.list_new}};
-  if (!P.loop_func || P.loop_threads != threads) {
-    int dev = 0, nsm = 0, occ = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    P.loop_smem = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, false);
-    // as many registers as the CTAs that shared memory lets an SM hold leave
-    const void* f = threads <= 384 ? (const void*)k_loop3d<56> : threads <= 512 ? (const void*)k_loop3d<64>
-                    : threads <= 768 ? (const void*)k_loop3d<80> : (const void*)k_loop3d<64>;
-    CK(raise_smem_limit(f, P.loop_smem));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, threads, P.loop_smem));
-    if (occ < 1) return "loop kernel cannot be resident (shared memory / registers)";
-    P.loop_func = f;
-    P.loop_threads = threads;
-    P.loop_grid = std::max(1, std::min(occ * nsm, L.nb));
-  }
   CK(cudaEventRecord(P.ev0, st));
   void* args[] = {&a, &s3};
-  CK(cudaLaunchCooperativeKernel(P.loop_func, dim3(P.loop_grid), dim3(threads), args, P.loop_smem, st));
+  CK(cudaLaunchCooperativeKernel(P.loop_func, dim3(P.loop_grid), dim3(P.loop_threads), args, P.loop_smem, st));
   return "";
 }
 
@@ -3483,12 +3509,17 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   // 2D solves of the reference's seven sweeps run in one resident kernel (k_loop2d)
   const bool loop2d = L.dim == 2 && sweeps == 7 && !opt.direct_launch && P.max_slots_pad <= 1024;
   // 3D ones of its two sweeps in another (k_loop3d)
-  const bool loop3d = visits && !P.prec && !opt.direct_launch;
-  if (!given && visits && (loop3d || P.prec)) {
+  bool loop3d = visits && !P.prec && !opt.direct_launch;
+  if (visits && (loop3d || P.prec)) {
     int dev = 0, nsm = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    threads = items_threads(L.nb, nsm, P.prec);
+    const int size = given ? threads : items_threads(L.nb, nsm, P.prec);
+    if (loop3d) {
+      std::string e = P.choose_loop3d(L, size, &loop3d);
+      if (!e.empty()) return e;
+    }
+    if (loop3d || P.prec) threads = size;
   }
   // per-instance iteration caps (one cap for all when not given)
   std::vector<int> cap(P.ninst, opt.max_iterations);
@@ -3522,7 +3553,7 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
     if (!e.empty()) return e;
     tele = opt.telemetry;
   } else if (loop3d) {
-    std::string e = P.run_loop3d(L, opt, cap, max_iters, hcap, threads);
+    std::string e = P.run_loop3d(L, opt, cap, max_iters, hcap);
     if (!e.empty()) return e;
     tele = opt.telemetry;
   } else {
