@@ -1247,8 +1247,8 @@ __global__ void __maxnreg__(EIK_ITEM_MAXNREG) k_sweep3d(DevArgs a) {
 // iteration's commit, then the active blocks; a candidate that moves is appended to this
 // iteration's active list and swept in the same visit.
 // ===========================================================================
-template <bool kPrec>
-__global__ void __maxnreg__(kPrec ? EIK_PREC_MAXNREG : EIK_ITEM_MAXNREG) k_items3d(DevArgs a) {
+template <bool kPrec, int kRegs>
+__global__ void __maxnreg__(kRegs) k_items3d(DevArgs a) {
   pdl_begin();
   extern __shared__ __align__(16) unsigned char sm[];
   __shared__ __align__(8) unsigned long long bar;
@@ -2974,7 +2974,10 @@ std::string DeviceSolve::Impl::build_graph(const Layout& L, int sweeps, int thre
         const size_t sv = smem_bytes_visit3d(P.max_slots_pad, P.max_local, P.max_owned, P.prec);
         if (sweeps == 2 && P.chk_memo && sv + 64 <= (size_t)maxsm) {
           items2 = true;
-          kv_fim = P.prec ? (void*)k_items3d<true> : (void*)k_items3d<false>;
+          // (an SM's 64 K registers give 1024 threads 64 each)
+          kv_fim = !P.prec           ? (void*)k_items3d<false, EIK_ITEM_MAXNREG>
+                   : threads <= 768 ? (void*)k_items3d<true, EIK_PREC_MAXNREG>
+                                    : (void*)k_items3d<true, 64>;
           vsmem = sv;
           a.chk_memo = P.chk_memo;
         }

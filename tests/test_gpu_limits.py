@@ -47,3 +47,24 @@ def test_blocks_at_the_shared_memory_limit(need_gpu, eik, mg, box, vpb, slots):
         assert e.stats()["max_slots_per_block"] == slots
     for other in got[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(got[0], other))
+
+
+def test_precision_mode_at_every_cta_size(need_gpu, eik, mg):
+    """A mesh with flagged tets; 1024 threads leave each 64 registers."""
+    xyz, tets = mg.kuhn_cube(13, 0.2, seed=4)
+    xyz[:, 2] = np.where(xyz[:, 2] > 0.5, xyz[:, 2] - 0.97 / 12 * np.minimum(1.0, (xyz[:, 2] - 0.5) * 12), xyz[:, 2])
+    metric = mg.anisotropic_metrics(tets.shape[0], seed=4)
+    got = []
+    for threads in (0, 128, 256, 384, 512, 768, 1024):
+        e = eik.Eikonal(False)
+        e.set_mesh(xyz, tets)
+        e.initSpeedMtxMultipliers(metric)
+        e.setSeeds([5, 1000])
+        e.maxIterations_ = 1000
+        e.keepHistory_ = 0
+        e.precisionMode_ = 1
+        e.threadsPerBlock_ = threads
+        got.append(outcome(e))
+        assert e.stats()["flagged_tets"] > 0
+    for other in got[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(got[0], other))
