@@ -373,8 +373,8 @@ def bench_batch(args, E, torch, world, local):
                      "kernel": "k_loop2d (the sweep phases of its iterations)",
                      "kernel_ms_per_step": fim_ms / args.steps},
         "clocks": clocks,
-        # one loop kernel per batch
-        "gpu_launches": args.steps,
+        # the loop kernel and k_publish, its control block to the host, per batch
+        "gpu_launches": 2 * args.steps,
     }
 
 
@@ -775,9 +775,10 @@ def main():
     fim_ms, chk_ms = st["fim_kernel_ms"] * args.steps, st["check_kernel_ms"] * args.steps
     fim_bytes = sum(launch_bytes(its, fused)[0]) * args.steps
     # one k_loop3d per solve; kernel by kernel the state initialisation (k_init_state,
-    # k_seed_state), then 3 kernels (sweep with checks, commit, close) or 4 per iteration
+    # k_seed_state), then 3 kernels (sweep with checks, commit, close) or 4 per iteration;
+    # behind either k_publish, the control block to the host
     one_launch = args.launch == "graph"
-    launches = args.steps * (1 if one_launch else 2 + (3 if fused else 4) * st["fim_launches"])
+    launches = args.steps * (2 if one_launch else 3 + (3 if fused else 4) * st["fim_launches"])
     e.telemetry_ = 0
     total_ms, upd_all = aggregate_replicas(torch, sum(times), upd, world, "cuda")
     value = upd_all / (total_ms * 1e-3)
