@@ -136,6 +136,20 @@ size_t device_footprint(const Layout& L, const Built3D* b = nullptr);
 // which then equals the host build's layout.
 std::string download_built(const Built3D& b, Layout& L);
 
+// A call that has work on a device's GPU while this object lives: a solve, a batch, a
+// server with running requests.  others(): how many such calls there were before it.
+class DeviceUse {
+ public:
+  explicit DeviceUse(int device);
+  ~DeviceUse();
+  DeviceUse(const DeviceUse&) = delete;
+  DeviceUse& operator=(const DeviceUse&) = delete;
+  int others() const { return others_; }
+
+ private:
+  int slot_, others_;
+};
+
 class DeviceSolve {
  public:
   DeviceSolve();
@@ -198,6 +212,7 @@ class DeviceSolve {
   volatile int* serve_pending() const;             // host side of the pending flag
   // Makes the device this object was created on current in the calling thread.
   void bind_thread() const;
+  int device() const;
   const SolveStats& stats() const { return stats_; }
   const Layout* layout() const { return L_; }
   void* stream() const { return stream_; }

@@ -46,6 +46,7 @@
 
 #include <algorithm>
 #include <cstdio>
+#include <atomic>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -2663,6 +2664,7 @@ struct DeviceSolve::Impl {
   int grid_visit = 0, grid_aux = 0;
   const void* loop_func = nullptr;  // loop kernel of the layout and its launch shape, chosen at its first solve
   int loop_grid = 0, loop_threads = 0;
+  long long loop_room = 0;  // CTAs of it that the GPU holds
   size_t loop_smem = 0;
   void* opt_stream = nullptr;  // the solver's stream
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -2715,7 +2717,17 @@ struct DeviceSolve::Impl {
   void fill_args(DevArgs& a, const Layout& L, int sweeps, int hcap, bool serve, bool tele) const;
   std::string build_graph(const Layout& L, int sweeps, int threads, int hcap, bool serve);
   std::string choose_loop2d(const Layout& L);
-  std::string choose_loop3d(const Layout& L, int threads, bool* resident);
+  std::string choose_loop3d(const Layout& L, int threads);
+  // Whether the loop kernel runs, `others` calls having work on the GPU.  Its CTAs stay
+  // for the whole solve and must all be resident, so a loop that fills the GPU keeps every
+  // other call waiting until it ends, where the graph's kernels take turns every few dozen
+  // microseconds.  It runs where as many loops of its size as there are calls fit together.
+  // Solves a second of 1 / 2 / 4 / 8 threads, loop against graph: 68 blocks of 160 threads
+  // (13 loops fit) 6030 / 10170 / 14580 / 18070 and 2730 / 4670 / 7850 / 13550; 160 blocks of
+  // 576 (one) 2710 / 3280 / 3240 / 3280 and 1340 / 2660 / 5220 / 9300; 245 3D blocks 1400 /
+  // 1250 / 1400 / 1380 and 1000 / 1650 / 3270 / 5310.  A request server's 32 requests beside a
+  // thread of 97^3 solves took 550 ms with the loop and 16 ms alone.
+  bool loop_runs(int others) const { return loop_grid > 0 && (others + 1ll) * loop_grid <= loop_room; }
   std::string stage_inputs(size_t o_words, const std::vector<int>& cap, int max_iters, int** words);
   std::string run_loop3d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap);
   std::string run_loop2d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap, int max_iters, int hcap);
@@ -2775,6 +2787,7 @@ void DeviceSolve::Impl::fill_args(DevArgs& a, const Layout& L, int sweeps, int h
 // Three lanes need blocks of at most 320 slots (1024 threads).
 std::string DeviceSolve::Impl::choose_loop2d(const Layout& L) {
   Impl& P = *this;
+  if (P.loop_func) return "";
   static const void* const resident[] = {(const void*)k_blocks2d<64>, (const void*)k_blocks2d<48>,
                                          (const void*)k_blocks2d<40>, (const void*)k_blocks2d<32>};
   const int threads[2] = {(L.max_slots + 9) / 10 * 32, (L.max_slots + 31) & ~31};
@@ -2790,6 +2803,7 @@ std::string DeviceSolve::Impl::choose_loop2d(const Layout& L) {
       P.loop_func = f;
       P.loop_threads = threads[0];
       P.loop_grid = L.nb;
+      P.loop_room = (long long)occ * nsm;
       return "";
     }
   // Three lanes per slot shorten a visit, one fills the GPU better.  A single solve's front
@@ -2811,14 +2825,14 @@ std::string DeviceSolve::Impl::choose_loop2d(const Layout& L) {
     CK(raise_smem_limit(f, P.loop_smem));
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, f, P.loop_threads, P.loop_smem));
   }
-  if (occ < 1) return "loop kernel cannot be resident (shared memory / registers)";
   P.loop_func = f;
-  P.loop_grid = std::max(1, std::min(occ * nsm, L.nb));
+  P.loop_grid = std::min(occ * nsm, std::max(L.nb, 1));
+  P.loop_room = (long long)occ * nsm;
   return "";
 }
 
-// One 2D solve or batch in k_loop2d, enqueued on the solver's stream: one copy of the
-// inputs, one launch.
+// One 2D solve or batch in its loop kernel (choose_loop2d), enqueued on the solver's stream:
+// one copy of the inputs, one launch.
 std::string DeviceSolve::Impl::run_loop2d(const Layout& L, const SolveOptions& opt, const std::vector<int>& cap,
                                           int max_iters, int hcap) {
   Impl& P = *this;
@@ -2838,17 +2852,16 @@ std::string DeviceSolve::Impl::run_loop2d(const Layout& L, const SolveOptions& o
             P.h_prev.empty() ? 0 : 1, a.ktime ? 1 : 0};
   if (!P.h_prev.empty())
     CK(cudaMemcpyAsync(P.prev, P.h_prev.data(), sizeof(float) * L.nv, cudaMemcpyHostToDevice, st));
-  if (!P.loop_func && !(e = P.choose_loop2d(L)).empty()) return e;
   CK(cudaEventRecord(P.ev0, st));
   void* args[] = {&a, &s2};
   CK(cudaLaunchCooperativeKernel(P.loop_func, dim3(P.loop_grid), dim3(P.loop_threads), args, P.loop_smem, st));
   return "";
 }
 
-// The 3D loop kernel of a layout and its launch shape at a CTA size; *resident: whether the
-// GPU holds a CTA of it.  (It keeps 200 bytes of its own where k_items3d keeps 32: blocks
+// The 3D loop kernel of a layout and its launch shape at a CTA size; loop_grid is 0 where
+// the GPU cannot hold a CTA of it.  (It keeps 200 bytes of its own where k_items3d keeps 32: blocks
 // of 3364 slots, 460 owned and 801 local vertices fit the one and not the other.)
-std::string DeviceSolve::Impl::choose_loop3d(const Layout& L, int threads, bool* resident) {
+std::string DeviceSolve::Impl::choose_loop3d(const Layout& L, int threads) {
   Impl& P = *this;
   if (!P.loop_func || P.loop_threads != threads) {
     int dev = 0, nsm = 0, occ = 0;
@@ -2869,8 +2882,8 @@ std::string DeviceSolve::Impl::choose_loop3d(const Layout& L, int threads, bool*
     P.loop_threads = threads;
     P.loop_smem = smem;
     P.loop_grid = std::min(occ * nsm, std::max(L.nb, 1));
+    P.loop_room = (long long)occ * nsm;
   }
-  *resident = P.loop_grid > 0;
   return "";
 }
 
@@ -3487,6 +3500,7 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
   Impl& P = *p_;
   if (!L_) return "no layout uploaded";
   const Layout& L = *L_;
+  const DeviceUse use(P.device);  // (counted until the results are there)
   cudaStream_t st = (cudaStream_t)stream_;
   const int sweeps = (opt.fim_sweeps > 0) ? opt.fim_sweeps : (L.dim == 3 ? 2 : 7);
   const bool given = opt.threads == 128 || opt.threads == 256 || opt.threads == 384 || opt.threads == 512 ||
@@ -3521,8 +3535,13 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
       }
     }
   }
-  // 2D solves of the reference's seven sweeps run in one resident kernel (k_loop2d)
-  const bool loop2d = L.dim == 2 && sweeps == 7 && !opt.direct_launch && P.max_slots_pad <= 1024;
+  // 2D solves of the reference's seven sweeps run in one resident kernel (choose_loop2d)
+  bool loop2d = L.dim == 2 && sweeps == 7 && !opt.direct_launch && P.max_slots_pad <= 1024;
+  if (loop2d) {
+    std::string e = P.choose_loop2d(L);
+    if (!e.empty()) return e;
+    loop2d = P.loop_runs(use.others());
+  }
   // 3D ones of its two sweeps in another (k_loop3d)
   bool loop3d = visits && !P.prec && !opt.direct_launch;
   if (visits && (loop3d || P.prec)) {
@@ -3531,8 +3550,9 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     const int size = given ? threads : items_threads(L.nb, nsm, P.prec);
     if (loop3d) {
-      std::string e = P.choose_loop3d(L, size, &loop3d);
+      std::string e = P.choose_loop3d(L, size);
       if (!e.empty()) return e;
+      loop3d = P.loop_runs(use.others());
     }
     if (loop3d || P.prec) threads = size;
   }
@@ -4157,6 +4177,16 @@ const float* DeviceSolve::serve_host_result(int inst) const {
 volatile int* DeviceSolve::serve_pending() const { return (volatile int*)p_->pending_host; }
 
 void DeviceSolve::bind_thread() const { cudaSetDevice(p_->device); }
+int DeviceSolve::device() const { return p_->device; }
+
+namespace {
+constexpr int kMaxDevices = 64;
+std::atomic<int> g_in_flight[kMaxDevices];
+}  // namespace
+DeviceUse::DeviceUse(int device) : slot_(device >= 0 && device < kMaxDevices ? device : kMaxDevices - 1) {
+  others_ = g_in_flight[slot_].fetch_add(1);
+}
+DeviceUse::~DeviceUse() { g_in_flight[slot_].fetch_sub(1); }
 
 std::string selftest_wait_timeout(int* status, double* waited_ms) {
   int* d_status = nullptr;
@@ -4305,6 +4335,7 @@ std::string solve3d_noalloc(const Layout& L, const std::vector<int>& seeds, int 
   const size_t smem = smem_bytes(ncoef, max_slots_pad, max_local, max_owned);
   int dev = 0, maxsm = 0, nsm = 0;
   CK(cudaGetDevice(&dev));
+  const DeviceUse use(dev);
   CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   if (smem + 64 > (size_t)maxsm) {

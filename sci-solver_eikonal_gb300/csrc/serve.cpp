@@ -160,11 +160,13 @@ void worker_loop(eik_server* S, int ai) {
   Arena& A = S->arenas[ai];
   A.dev->bind_thread();
   std::vector<int> done, iters;
+  std::unique_ptr<DeviceUse> use;  // while requests run
   for (;;) {
     std::vector<Admission> adm;
     std::vector<int> cancel;
     {
       std::unique_lock<std::mutex> lk(S->mu);
+      if (A.running.empty() && !has_admissible(S, ai)) use.reset();
       S->cv_work.wait(lk, [&] { return S->stop || !A.running.empty() || has_admissible(S, ai); });
       if (S->stop) return;
       for (auto& kv : A.running)
@@ -196,6 +198,7 @@ void worker_loop(eik_server* S, int ai) {
       }
       *A.pending = 0;
     }
+    if (!use) use.reset(new DeviceUse(A.dev->device()));
     std::string e;
     const auto r0 = std::chrono::steady_clock::now();
     if (!cancel.empty()) e = A.dev->serve_cancel(cancel);
