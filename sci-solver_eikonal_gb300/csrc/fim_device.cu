@@ -2597,6 +2597,7 @@ struct DeviceSolve::Impl {
   std::vector<unsigned char> h_stage;
   Ctl* last_ctl = nullptr;  // the control block of the last solve
   Ctl* h_ctl = nullptr;     // its copy on the host (pinned and mapped)
+  bool solved_before = false;
   int* cand = nullptr;        // 2 x nb check candidates (checks inside the sweep kernel)
   int* inst_swept = nullptr;  // per instance: blocks swept this iteration
   int* inst_ncand = nullptr;  // per instance: check candidates queued this iteration
@@ -3716,11 +3717,19 @@ std::string DeviceSolve::solve(const SolveOptions& opt) {
     }
   }
   CK(cudaEventRecord(P.ev1, st));
-  if (!P.h_ctl) CK(cudaHostAlloc((void**)&P.h_ctl, sizeof(Ctl), cudaHostAllocMapped));
-  k_publish<<<1, 32, 0, st>>>(P.last_ctl, P.h_ctl);
+  // (a handle's first solve, often its only one, copies behind the wait: pinned memory takes
+  // 180 us to get and give back)
+  const bool publish = P.solved_before;
+  if (publish) {
+    if (!P.h_ctl) CK(cudaHostAlloc((void**)&P.h_ctl, sizeof(Ctl), cudaHostAllocMapped));
+    k_publish<<<1, 32, 0, st>>>(P.last_ctl, P.h_ctl);
+  }
   CK(cudaStreamSynchronize(st));
   CK(cudaGetLastError());
-  Ctl out = *P.h_ctl;
+  Ctl out{};
+  if (publish) out = *P.h_ctl;
+  else CK(cudaMemcpy(&out, P.last_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost));
+  P.solved_before = true;
   if (out.bar.fail) out.error |= kErrWait;
   cudaEventElapsedTime(&stats_.solve_ms, P.ev0, P.ev1);
   // a trailing iteration that swept nothing (its checks activated no block) is not
