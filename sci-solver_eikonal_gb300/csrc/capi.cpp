@@ -882,8 +882,12 @@ struct eik_batch {
   std::vector<std::string> keys;  // per handle: layout identity at pack time
   Layout layout;
   std::unique_ptr<DeviceSolve> dev;
-  bool packed = false, solved = false, have_host = false;
+  bool packed = false, solved = false;
+  // the last solve's results: in host_result (have_host), on the device (on_device) or both;
+  // vbeg: their instances' ranges; fetched: handed out since; ranged: one instance's alone
+  bool have_host = false, on_device = false, fetched = false, ranged = false;
   std::vector<float> host_result;
+  std::vector<int> vbeg;
   std::vector<int> iters;
   eik_stats stats{};
   std::string err;
@@ -894,6 +898,16 @@ namespace {
 int bfail(eik_batch* b, int code, const std::string& msg) {
   if (b) b->err = msg;
   return code;
+}
+
+// Copies the last solve's results into host_result.
+int keep_results(eik_batch* b) {
+  if (!b->on_device) return bfail(b, EIK_ERR_STATE, "a later solve that failed has replaced the results");
+  b->host_result.resize((size_t)b->vbeg.back());
+  std::string e = b->dev->result(b->host_result.data());
+  if (!e.empty()) return bfail(b, EIK_ERR_CUDA, e);
+  b->have_host = true;
+  return EIK_OK;
 }
 
 std::string layout_identity(const eik_solver* h) {
@@ -1045,6 +1059,9 @@ int eik_batch_solve(eik_batch* b) {
   }
   if (repack) {
     b->packed = false;
+    // results that were read stay readable if this solve fails behind here
+    if (b->solved && b->fetched && !b->have_host) (void)keep_results(b);
+    b->on_device = false;
     std::string e;
     if (on_device) {
       e = batch_device_pack(b);
@@ -1072,10 +1089,11 @@ int eik_batch_solve(eik_batch* b) {
   so.inst_max_iterations.resize(n);
   for (int i = 0; i < n; ++i) so.inst_max_iterations[i] = b->solvers[i]->opt.max_iterations;
   b->solved = false;
-  b->have_host = false;
+  b->have_host = b->on_device = b->fetched = b->ranged = false;
   e = b->dev->solve(so);
   if (!e.empty()) return bfail(b, b->dev->stats().error ? EIK_ERR_DEVICE : EIK_ERR_CUDA, e);
-  b->solved = true;
+  b->solved = b->on_device = true;
+  b->vbeg = b->layout.inst_vbeg;
   b->iters = b->dev->stats().inst_iters;
   fill_stats(b->stats, b->dev->stats(), b->layout, std::chrono::duration<float, std::milli>(t1 - t0).count());
   return EIK_OK;
@@ -1096,27 +1114,33 @@ int eik_batch_num_iterations(const eik_batch* b, int i) {
 int eik_batch_get_results(eik_batch* b, float* out, long long n) {
   if (!b || !out) return EIK_ERR_ARG;
   if (!b->solved) return bfail(b, EIK_ERR_STATE, "no batch solve yet");
-  if (n != b->layout.nv) return bfail(b, EIK_ERR_ARG, "size mismatch");
+  if (n != b->vbeg.back()) return bfail(b, EIK_ERR_ARG, "size mismatch");
+  if (!b->on_device && !b->have_host) return keep_results(b);
   if (b->have_host) {
     std::memcpy(out, b->host_result.data(), sizeof(float) * (size_t)n);
   } else {  // straight into the caller's array
     std::string e = b->dev->result(out);
     if (!e.empty()) return bfail(b, EIK_ERR_CUDA, e);
   }
+  b->fetched = true;
   return EIK_OK;
 }
 
 int eik_batch_get_result(eik_batch* b, int i, float* out, int nv) {
   if (!b || !out || i < 0 || i >= (int)b->solvers.size()) return EIK_ERR_ARG;
   if (!b->solved) return bfail(b, EIK_ERR_STATE, "no batch solve yet");
-  const int v0 = b->layout.inst_vbeg[i], cnt = b->layout.inst_vbeg[i + 1] - v0;
+  const int v0 = b->vbeg[i], cnt = b->vbeg[i + 1] - v0;
   if (nv != cnt) return bfail(b, EIK_ERR_ARG, "size mismatch");
-  if (!b->have_host) {
-    b->host_result.resize(b->layout.nv);
-    std::string e = b->dev->result(b->host_result.data());
+  if (b->on_device && b->fetched && !b->have_host && !b->ranged) {
+    // one instance behind all of them: its own range; from the second on they are kept
+    b->ranged = true;
+    std::string e = b->dev->result_range(v0, cnt, out);
     if (!e.empty()) return bfail(b, EIK_ERR_CUDA, e);
-    b->have_host = true;
+    return EIK_OK;
   }
+  if (!b->have_host)
+    if (int rc = keep_results(b)) return rc;
+  b->fetched = true;
   std::memcpy(out, b->host_result.data() + v0, sizeof(float) * (size_t)cnt);
   return EIK_OK;
 }
@@ -1124,7 +1148,8 @@ int eik_batch_get_result(eik_batch* b, int i, float* out, int nv) {
 int eik_batch_get_results_device(eik_batch* b, float* out_dev, long long n) {
   if (!b || !out_dev) return EIK_ERR_ARG;
   if (!b->solved) return bfail(b, EIK_ERR_STATE, "no batch solve yet");
-  if (n != b->layout.nv) return bfail(b, EIK_ERR_ARG, "size mismatch");
+  if (n != b->vbeg.back()) return bfail(b, EIK_ERR_ARG, "size mismatch");
+  if (!b->on_device) return bfail(b, EIK_ERR_STATE, "a later solve that failed has replaced the results");
   std::string e = b->dev->result_device(out_dev);
   if (!e.empty()) return bfail(b, EIK_ERR_CUDA, e);
   return EIK_OK;

@@ -187,6 +187,7 @@ class DeviceSolve {
   std::string solve(const SolveOptions& opt);
   // Final travel times in original vertex order.
   std::string result(float* out_host) const;
+  std::string result_range(int v0, int n, float* out_host) const;  // n of them from vertex v0 on
   std::string result_device(float* out_dev) const;  // device pointer, original order
   std::string history(int i, float* out_host) const;
   // One visit of every block with the 2D kernel on the given vertex values

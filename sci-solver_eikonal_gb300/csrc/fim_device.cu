@@ -3831,6 +3831,19 @@ std::string DeviceSolve::result(float* out_host) const {
   return "";
 }
 
+std::string DeviceSolve::result_range(int v0, int n, float* out_host) const {
+  const Impl& P = *p_;
+  if (!L_ || v0 < 0 || n < 0 || v0 > P.nv - n) return "range outside the layout";
+  if (n == 0) return "";
+  cudaStream_t st = (cudaStream_t)stream_;
+  k_gather_result<<<std::max(1, std::min(1024, (n + 255) / 256)), 256, 0, st>>>(P.Ta, P.visited, P.vblock, P.perm + v0,
+                                                                               n, P.dim, P.out_tmp);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(out_host, P.out_tmp, sizeof(float) * n, cudaMemcpyDeviceToHost, st));
+  CK(cudaStreamSynchronize(st));
+  return "";
+}
+
 std::string DeviceSolve::history(int i, float* out_host) const {
   const Impl& P = *p_;
   if (!P.hist || i < 0 || i >= P.hist_cap || i >= stats_.iterations) return "iteration not recorded";

@@ -158,3 +158,48 @@ def test_batch_device_build_equals_host_build(need_gpu, eik, mg, dim):
         e.deviceSetup_ = 1
         res, it = _alone(e)
         assert it == runs[1][1][i] and bits_equal(res, runs[1][0][i]), i
+
+
+@pytest.mark.parametrize("device_setup", [1, 0])
+def test_results_outlive_a_solve_that_is_refused(need_gpu, eik, mg, device_setup):
+    """Results that were read can be read again, all of them and one by one, also behind a
+    later solve that fails because a handle's blocks have become too large; results that
+    were never read are then refused."""
+    hs = [_cube_solver(eik, mg, n, n, [n]) for n in (9, 17, 13)]
+    for h in hs:
+        h.deviceSetup_ = device_setup
+    want = [_alone(h)[0] for h in hs]
+    b = eik.EikonalBatch(hs)
+
+    def reads():
+        for _ in range(2):
+            assert all(bits_equal(g, w) for g, w in zip(b.getFinalResults(), want))
+        for i in (1, 0, 2, 1):
+            assert bits_equal(b.getFinalResult(i), want[i])
+        assert all(bits_equal(g, w) for g, w in zip(b.getFinalResults(), want))
+
+    for one_first in (False, True):
+        b.solveEikonal()
+        if one_first:
+            assert bits_equal(b.getFinalResult(2), want[2])
+        reads()
+    b.solveEikonal()
+    assert all(bits_equal(g, w) for g, w in zip(b.getFinalResults(), want))  # read once, then refused
+    hs[1].maxVertsPerBlock_ = 5000
+    for _ in range(2):
+        with pytest.raises(eik.EikonalError) as ex:
+            b.solveEikonal()
+        assert "shared memory" in str(ex.value)
+        reads()
+    hs[1].maxVertsPerBlock_ = 64
+    b.solveEikonal()
+    hs[1].maxVertsPerBlock_ = 5000
+    with pytest.raises(eik.EikonalError):
+        b.solveEikonal()
+    with pytest.raises(eik.EikonalError):
+        b.getFinalResults()
+    with pytest.raises(eik.EikonalError):
+        b.getFinalResult(0)
+    hs[1].maxVertsPerBlock_ = 64
+    b.solveEikonal()
+    reads()
