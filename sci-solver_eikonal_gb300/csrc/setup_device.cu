@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "device.hpp"
+#include "scratch.hpp"
 
 namespace eikgb {
 namespace {
@@ -453,32 +454,20 @@ __global__ void k_live2d(const int* ekey, const unsigned long long* eval, const 
 }
 
 // temporary device buffers of one build, freed on every exit
-// Working arrays of one build, carved from a few large pieces (each at least as large as
-// all before it) that are freed together: the build of a 33^3 cube asked for 45 arrays,
-// whose allocation and release one by one took 1.2 ms of its 2.5.
-struct Scratch {
-  std::vector<void*> pieces;
-  unsigned char* at = nullptr;
-  size_t left = 0, total = 0;
-  ~Scratch() {
-    for (void* p : pieces) cudaFree(p);
+struct DeviceAlloc {
+  bool get(void** p, size_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    (void)cudaGetLastError();  // a smaller request may follow
+    return false;
   }
+  void put(void* p) { cudaFree(p); }
+};
+struct Scratch {
+  ScratchPieces<DeviceAlloc> pieces;
   template <typename T>
   std::string get(T*& p, size_t n) {
-    p = nullptr;
-    const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
-    if (bytes > left) {
-      const size_t piece = std::max(bytes, std::max<size_t>(total, (size_t)8 << 20));
-      void* q = nullptr;
-      CKS(cudaMalloc(&q, piece));
-      pieces.push_back(q);
-      at = static_cast<unsigned char*>(q);
-      left = piece;
-      total += piece;
-    }
-    p = reinterpret_cast<T*>(at);
-    at += bytes;
-    left -= bytes;
+    p = static_cast<T*>(pieces.get(std::max<size_t>(n, 1) * sizeof(T)));
+    if (!p) return "device set-up: out of memory for " + std::to_string(n * sizeof(T)) + " bytes of working memory";
     return "";
   }
 };
