@@ -8,6 +8,7 @@
 #include <cstring>
 #include <numeric>
 #include <set>
+#include <system_error>
 #include <thread>
 
 namespace eikgb {
@@ -337,9 +338,15 @@ void rcb(RcbPoint* p, int n, int nparts, int first, int* labels, int depth) {
   // the two halves are independent: the first levels run them on two threads
   // (a thread takes about 20 us to start, 4096 points about 100 us to split up)
   if (depth < 4 && n >= 4096) {
-    std::thread left([=] { rcb(p, nl, pl, first, labels, depth + 1); });
+    const auto left = [=] { rcb(p, nl, pl, first, labels, depth + 1); };
+    std::thread t;
+    try {
+      t = std::thread(left);
+    } catch (const std::system_error&) {  // no thread to be had (a limit of the process or the system)
+    }
     rcb(p + nl, n - nl, nparts - pl, first + pl, labels, depth + 1);
-    left.join();
+    if (t.joinable()) t.join();
+    else left();
   } else {
     rcb(p, nl, pl, first, labels, depth + 1);
     rcb(p + nl, n - nl, nparts - pl, first + pl, labels, depth + 1);
