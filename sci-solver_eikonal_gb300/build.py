@@ -30,7 +30,7 @@ NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", *ARCH, "-Xcompiler", "-fPIC", "-
 HOST_SRC = ["setup.cpp", "mesh_io.cpp", "capi.cpp", "serve.cpp"]
 CUDA_SRC = ["fim_device.cu", "setup_device.cu"]
 HEADERS = ["setup.hpp", "mesh_io.hpp", "device.hpp", "local_update.cuh", "loop2d.cuh", "visit3d.cuh", "loop3d.cuh",
-           "scratch.hpp", "solver_access.hpp"]
+           "scratch.hpp", "visit_sum.hpp", "solver_access.hpp"]
 
 
 def _metis_archive():

@@ -54,6 +54,7 @@
 #include <vector>
 
 #include "device.hpp"
+#include "visit_sum.hpp"
 #include "local_update.cuh"
 
 namespace eikgb {
@@ -2860,7 +2861,7 @@ std::string DeviceSolve::Impl::run_loop2d(const Layout& L, const SolveOptions& o
 }
 
 // The 3D loop kernel of a layout and its launch shape at a CTA size; loop_grid is 0 where
-// the GPU cannot hold a CTA of it.  (It keeps 200 bytes of its own where k_items3d keeps 32: blocks
+// the GPU cannot hold a CTA of it.  (It keeps 300 bytes of its own where k_items3d keeps 32: blocks
 // of 3364 slots, 460 owned and 801 local vertices fit the one and not the other.)
 std::string DeviceSolve::Impl::choose_loop3d(const Layout& L, int threads) {
   Impl& P = *this;

@@ -490,11 +490,12 @@ __global__ void __maxnreg__(kRegs) k_loop2d(DevArgs a, Start2 st) {
   int iter = 0, nact = st.nact;
   bool go = nact > 0 && a.ctl->max_iters > 0;
   const int cap0 = st.maxit[0];
-  // thread 0's counts, added to the solve's at the end (per-visit atomics of a batch's
-  // thousands of visits met at the same addresses): visits, slots, halo and owned
-  // vertices of the sweeps, then of the checks
-  __shared__ unsigned s_cnt[8];
-  if (tid < 8) s_cnt[tid] = 0u;
+  // thread 0's sums, added to the solve's at the end
+  __shared__ VisitSum s_swept, s_checked;
+  if (tid == 0) {
+    s_swept.clear();
+    s_checked.clear();
+  }
   // the CTA's present and next item: words 0-7 the block's descriptor, 8 and 9 its range of
   // neighbours, 10 its instance, 11 the block, 12 whether the instance is finished
   __shared__ int s_item[2][16];
@@ -578,10 +579,7 @@ __global__ void __maxnreg__(kRegs) k_loop2d(DevArgs a, Start2 st) {
         }
       }
       if (tid == 0) {
-        s_cnt[0] += 1u;
-        s_cnt[1] += bd.nslots;
-        s_cnt[2] += bd.nhalo;
-        s_cnt[3] += bd.nowned;
+        s_swept.add(bd.nslots, bd.nhalo, bd.nowned);
         if (st.telemetry) count_visit(a, iter, 0, bd.nslots, bd.nhalo, bd.nowned);
       }
     }
@@ -643,10 +641,7 @@ __global__ void __maxnreg__(kRegs) k_loop2d(DevArgs a, Start2 st) {
           if (!single) atomicAdd(&a.inst_nnext[inst], 1);
           a.stampA[b] = stamp + 1;  // member of the next iteration's active list
         }
-        s_cnt[4] += 1u;
-        s_cnt[5] += bd.nslots;
-        s_cnt[6] += bd.nhalo;
-        s_cnt[7] += bd.nowned;
+        s_checked.add(bd.nslots, bd.nhalo, bd.nowned);
         if (st.telemetry) count_visit(a, iter, 1, bd.nslots, bd.nhalo, bd.nowned);
       }
     }
@@ -677,20 +672,19 @@ __global__ void __maxnreg__(kRegs) k_loop2d(DevArgs a, Start2 st) {
       c->iter = iter;
       a.inst_iters[0] = iter;
     }
-    const unsigned long long f[4] = {s_cnt[0], s_cnt[1], s_cnt[2], s_cnt[3]};
-    const unsigned long long h[4] = {s_cnt[4], s_cnt[5], s_cnt[6], s_cnt[7]};
-    if (f[0]) {
-      atomicAdd(&c->fim_visits, f[0]);
-      atomicAdd(&c->fim_slots, f[1]);
-      atomicAdd(&c->fim_halo, f[2]);
-      atomicAdd(&c->fim_owned, f[3]);
+    const VisitSum f = s_swept, h = s_checked;
+    if (f.visits) {
+      atomicAdd(&c->fim_visits, f.visits);
+      atomicAdd(&c->fim_slots, f.slots);
+      atomicAdd(&c->fim_halo, f.halo);
+      atomicAdd(&c->fim_owned, f.owned);
     }
-    if (h[0]) atomicAdd(&c->chk_visits, h[0]);
-    if (f[0] + h[0]) {
-      atomicAdd(&c->updates, 7ull * f[3] + h[3]);
-      atomicAdd(&c->slot_visits, f[1] + h[1]);
-      atomicAdd(&c->halo_visits, f[2] + h[2]);
-      atomicAdd(&c->owned_visits, f[3] + h[3]);
+    if (h.visits) atomicAdd(&c->chk_visits, h.visits);
+    if (f.visits + h.visits) {
+      atomicAdd(&c->updates, 7ull * f.owned + h.owned);
+      atomicAdd(&c->slot_visits, f.slots + h.slots);
+      atomicAdd(&c->halo_visits, f.halo + h.halo);
+      atomicAdd(&c->owned_visits, f.owned + h.owned);
     }
   }
 }

@@ -170,7 +170,8 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
   __shared__ volatile Item3 s_it[2];
   __shared__ int s_n[2];
   __shared__ volatile int s_moved;
-  __shared__ unsigned s_cnt[12];  // visits, slots, halo, owned of sweeps, checks and sweeps behind a check
+  __shared__ PassSum s_swept, s_checked, s_both;  // s_both: sweeps behind a check
+  __shared__ VisitSum s_sum[3];                   // the same over the solve
   const SmemV s = carve_visit3d<false>(sm, a);
   GridBar* const g = &a.ctl->bar;
   const int tid = threadIdx.x, lane = tid & 31, NT = blockDim.x;
@@ -203,7 +204,12 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
   // ---- initial state ----
   if (tid == 0) mbar_init(&bar, 1);
   if (tid < 2) s_n[tid] = 0;
-  if (tid < 12) s_cnt[tid] = 0u;
+  if (tid == 0) {
+    s_swept.clear();
+    s_checked.clear();
+    s_both.clear();
+    for (VisitSum& x : s_sum) x.clear();
+  }
   for (int i = gtid; i < a.nv; i += gn) a.Ta[i] = a.Tb[i] = kLarge3DDev;
   for (int b = gtid; b < a.nb; b += gn) {
     a.stampA[b] = st.queued[0][b] = st.queued[1][b] = 0;
@@ -277,10 +283,7 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
           if (sweep) sweep_visit3d(a, bd, s, s_n, chk, (it.flags & 4) != 0);
         }
         if (chk && tid == 0) {
-          s_cnt[4] += 1u;
-          s_cnt[5] += it.bd.nslots;
-          s_cnt[6] += it.bd.nhalo;
-          s_cnt[7] += it.bd.nowned;
+          s_checked.add(it.bd.nslots, it.bd.nhalo, it.bd.nowned);
           count_visit(a, v.iter - 1, 1, it.bd.nslots, it.bd.nhalo, it.bd.nowned);
           if (sweep) atomicAdd(&st.turn[v.iter % 3].add, 1);
         }
@@ -317,16 +320,10 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
             atomicAdd(&a.inst_swept[a.blk_inst[b]], 1);
             if (!allc) atomicAdd(&a.inst_nnext[a.blk_inst[b]], 1);
           }
-          s_cnt[0] += 1u;
-          s_cnt[1] += it.bd.nslots;
-          s_cnt[2] += it.bd.nhalo;
-          s_cnt[3] += nown;
+          s_swept.add(it.bd.nslots, it.bd.nhalo, nown);
           count_visit(a, iter, 0, it.bd.nslots, it.bd.nhalo, nown);
           if (chk) {  // streamed once, with the check
-            s_cnt[8] += 1u;
-            s_cnt[9] += it.bd.nslots;
-            s_cnt[10] += it.bd.nhalo;
-            s_cnt[11] += nown;
+            s_both.add(it.bd.nslots, it.bd.nhalo, nown);
             count_visit(a, iter, 2, it.bd.nslots, it.bd.nhalo, nown);
           }
         }
@@ -359,6 +356,11 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
     copy_settled(a, st.conv + (size_t)((v.iter + 1) & 1) * a.nb, v.nconv, st.queued[(v.iter + 1) & 1], v.iter,
                  buf_in(a, v.iter), buf_out(a, v.iter));
     if (v.snap >= 0 && v.snap < a.hist_cap) snapshot3d(a, v.snap, v.iter + 1, buf_in(a, v.iter));
+    if (tid == 0 && v.iter % kTakeEvery == kTakeEvery - 1) {
+      take(s_sum[0], s_swept, false);
+      take(s_sum[1], s_checked, false);
+      take(s_sum[2], s_both, false);
+    }
     // ---- close ----
     if (!sync_grid([&] {
           if (!single) finish_loop3d(a, v.iter);
@@ -407,20 +409,22 @@ __global__ void __maxnreg__(kRegs) k_loop3d(const __grid_constant__ DevArgs a,
       c->iter = iter;
       a.inst_iters[0] = v.iters;
     }
-    unsigned long long n[12];
-    for (int i = 0; i < 12; ++i) n[i] = s_cnt[i];
-    if (n[0]) {
-      atomicAdd(&c->fim_visits, n[0]);
-      atomicAdd(&c->fim_slots, n[1]);
-      atomicAdd(&c->fim_halo, n[2]);
-      atomicAdd(&c->fim_owned, n[3]);
+    take(s_sum[0], s_swept, true);
+    take(s_sum[1], s_checked, true);
+    take(s_sum[2], s_both, true);
+    const VisitSum f = s_sum[0], h = s_sum[1], x = s_sum[2];
+    if (f.visits) {
+      atomicAdd(&c->fim_visits, f.visits);
+      atomicAdd(&c->fim_slots, f.slots);
+      atomicAdd(&c->fim_halo, f.halo);
+      atomicAdd(&c->fim_owned, f.owned);
     }
-    if (n[4]) atomicAdd(&c->chk_visits, n[4]);
-    if (n[0] + n[4]) {  // a block swept behind its check was streamed once
-      atomicAdd(&c->updates, 2ull * n[3] + n[7]);
-      atomicAdd(&c->slot_visits, n[1] + n[5] - n[9]);
-      atomicAdd(&c->halo_visits, n[2] + n[6] - n[10]);
-      atomicAdd(&c->owned_visits, n[3] + n[7] - n[11]);
+    if (h.visits) atomicAdd(&c->chk_visits, h.visits);
+    if (f.visits + h.visits) {  // a block swept behind its check was streamed once
+      atomicAdd(&c->updates, 2ull * f.owned + h.owned);
+      atomicAdd(&c->slot_visits, f.slots + h.slots - x.slots);
+      atomicAdd(&c->halo_visits, f.halo + h.halo - x.halo);
+      atomicAdd(&c->owned_visits, f.owned + h.owned - x.owned);
     }
   }
 }

@@ -26,7 +26,7 @@ def outcome(e):
 
 @pytest.mark.parametrize("box,vpb,slots", [
     ((14, 19, 19), 440, 3074),
-    ((14, 19, 19), 460, 3364),  # the visit's state fits, beside the loop kernel's own 200 bytes it does not
+    ((14, 19, 19), 460, 3364),  # the visit's state fits, beside what the loop kernel keeps itself it does not
     ((14, 19, 21), 468, 3362),
 ])
 def test_blocks_at_the_shared_memory_limit(need_gpu, eik, mg, box, vpb, slots):
