@@ -258,6 +258,12 @@ int eik_selftest_local_update(int which, const float* in, float* out, int n);
  * waited_ms (may be null) receives how long it waited. */
 int eik_selftest_wait_timeout(double* waited_ms);
 
+/* The same of the grid barrier at which a loop kernel's CTAs meet: CTAs wait, for one
+ * second here and for four in a solve, for arrivals that never come, give up and raise
+ * the barrier's flag; a second launch finds it raised.  EIK_ERR_DEVICE when all of them
+ * gave up; the longest wait of either launch in waited_ms and next_ms (may be null). */
+int eik_selftest_grid_wait(double* waited_ms, double* next_ms);
+
 /* Allocation-free 3D solve.  No counterpart in the reference: an addition for
  * callers that cannot call cudaMalloc, such as code running while another
  * component captures the stream into a CUDA graph, real-time or embedded hosts

@@ -117,6 +117,7 @@ SIGNATURES = {
     "eik_selftest_local_update": (ctypes.c_int, [ctypes.c_int, _FP, _FP, ctypes.c_int]),
     "eik_stream": (_P, [_P]),
     "eik_selftest_wait_timeout": (ctypes.c_int, [ctypes.POINTER(ctypes.c_double)]),
+    "eik_selftest_grid_wait": (ctypes.c_int, [ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_double)]),
     "eik_solve3d_noalloc": (ctypes.c_int, [_FP, ctypes.c_int, _IP, ctypes.c_int, _FP, ctypes.c_longlong, _IP,
                                            ctypes.c_int, ctypes.c_int, ctypes.c_int, _FP, _P, _IP, ctypes.c_char_p,
                                            ctypes.c_int]),
@@ -599,6 +600,14 @@ def selftest_wait_timeout():
     ms = ctypes.c_double()
     rc = lib().eik_selftest_wait_timeout(ctypes.byref(ms))
     return rc, ms.value
+
+
+def selftest_grid_wait():
+    """The same of the loop kernels' grid barrier: (status code, waited ms, waited ms of
+    CTAs that find it given up)."""
+    ms, later = ctypes.c_double(), ctypes.c_double()
+    rc = lib().eik_selftest_grid_wait(ctypes.byref(ms), ctypes.byref(later))
+    return rc, ms.value, later.value
 
 
 def solve3d_noalloc(xyz, tets, speeds=None, seeds=(0,), max_verts_per_block=64, max_iterations=100, stream=0):

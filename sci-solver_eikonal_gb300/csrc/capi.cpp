@@ -753,6 +753,15 @@ int eik_selftest_wait_timeout(double* waited_ms) {
   return status ? EIK_ERR_DEVICE : EIK_OK;
 }
 
+int eik_selftest_grid_wait(double* waited_ms, double* next_ms) {
+  int status = 0;
+  double ms = 0, next = 0;
+  if (!selftest_grid_wait(&status, &ms, &next).empty()) return EIK_ERR_CUDA;
+  if (waited_ms) *waited_ms = ms;
+  if (next_ms) *next_ms = next;
+  return status ? EIK_ERR_DEVICE : EIK_OK;
+}
+
 int eik_selftest_local_update(int which, const float* in, float* out, int n) {
   if (which < 0 || which > 7 || n < 0 || (n > 0 && (!in || !out))) return EIK_ERR_ARG;
   return selftest_device(which, in, out, n).empty() ? EIK_OK : EIK_ERR_CUDA;

@@ -237,6 +237,11 @@ std::string selftest_device(int which, const float* in, float* out, int n);
 // the device error flag (nonzero when the wait gave up), waited_ms its duration.
 std::string selftest_wait_timeout(int* status, double* waited_ms);
 
+// The same of the loop kernels' grid barrier: CTAs that wait for arrivals which never
+// come give up and raise the barrier's flag (waited_ms), at which later waits end
+// (next_ms).
+std::string selftest_grid_wait(int* status, double* waited_ms, double* next_ms);
+
 // Allocation-free 3D solve: the layout and every solver buffer live in a fixed
 // 32 MiB array of the library's device image (no cudaMalloc / cudaFree).  Runs on
 // `stream` (a cudaStream_t, may be null), one host round trip per outer

@@ -2408,6 +2408,17 @@ __global__ void k_selftest_wait(int* status, unsigned long long* waited_ns) {
   }
 }
 
+// the same of the grid barrier's wait: CTAs that wait for one more than there are.  Each
+// ends by itself, whether or not the others run.
+__global__ void k_selftest_grid_wait(GridBar* g, unsigned limit_ms, int* status, unsigned long long* waited_ns) {
+  if (threadIdx.x != 0) return;
+  (void)grid_arrive(&g->count, 0u);
+  const unsigned long long t0 = global_ns();
+  const bool ok = grid_wait(g, &g->count, 2u * gridDim.x, limit_ms * 1000000ull);
+  waited_ns[blockIdx.x] = global_ns() - t0;
+  status[blockIdx.x] = ok ? 0 : kErrWait;
+}
+
 __global__ void k_selftest_tet(const float* in, float* out, int n) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
@@ -4225,6 +4236,37 @@ std::string selftest_wait_timeout(int* status, double* waited_ms) {
   cudaFree(d_ns);
   if (e != cudaSuccess) return std::string("wait self-test: ") + cudaGetErrorString(e);
   *waited_ms = (double)ns * 1e-6;
+  return "";
+}
+
+std::string selftest_grid_wait(int* status, double* waited_ms, double* next_ms) {
+  constexpr int kCtas = 4;
+  struct Out {
+    GridBar g;
+    int status[kCtas];
+    unsigned long long ns[kCtas];
+  } h{};
+  Out* d = nullptr;
+  CK(cudaMalloc((void**)&d, sizeof(Out)));
+  cudaError_t e = cudaSuccess;
+  *status = kErrWait;
+  for (int run = 0; run < 2 && e == cudaSuccess; ++run) {
+    // the second run's CTAs find the flag that the first one's raised
+    h.g.count = 0;
+    e = cudaMemcpy(d, &h, sizeof(Out), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) break;
+    k_selftest_grid_wait<<<kCtas, 32>>>(&d->g, 1000u, d->status, d->ns);
+    e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = cudaMemcpy(&h, d, sizeof(Out), cudaMemcpyDeviceToHost);
+    double most = 0;
+    for (int i = 0; i < kCtas; ++i) {
+      most = std::max(most, (double)h.ns[i] * 1e-6);
+      if (h.status[i] != kErrWait || h.g.fail != 1u) *status = 0;
+    }
+    *(run ? next_ms : waited_ms) = most;
+  }
+  cudaFree(d);
+  if (e != cudaSuccess) return std::string("grid wait self-test: ") + cudaGetErrorString(e);
   return "";
 }
 

@@ -58,7 +58,8 @@ __device__ __forceinline__ bool grid_arrive(unsigned* count, unsigned want) {
   return old + 1u == want;
 }
 // thread 0: waits until *word reaches `want`
-__device__ __forceinline__ bool grid_wait(GridBar* g, const unsigned* word, unsigned want) {
+__device__ __forceinline__ bool grid_wait(GridBar* g, const unsigned* word, unsigned want,
+                                          unsigned long long limit_ns = kGridWaitNs) {
   unsigned long long t0 = 0;
   for (unsigned i = 0;; ++i) {
     if ((int)(ld_acquire(word) - want) >= 0) return true;
@@ -67,7 +68,7 @@ __device__ __forceinline__ bool grid_wait(GridBar* g, const unsigned* word, unsi
       if (ld_acquire(&g->fail)) return false;
       const unsigned long long t = global_ns();
       if (t0 == 0) t0 = t;
-      if (t - t0 > kGridWaitNs) {
+      if (t - t0 > limit_ns) {
         st_release(&g->fail, 1u);
         return false;
       }

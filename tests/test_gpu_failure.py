@@ -28,6 +28,21 @@ def test_bounded_wait_gives_up_and_the_context_stays_usable(need_gpu, eik, golde
     assert r[0] == 0.0 and np.all(np.abs(r[1:] - np.float32(19.58)) <= 4 * np.spacing(np.float32(19.58)))
 
 
+def test_grid_barrier_gives_up_and_the_context_stays_usable(need_gpu, eik, mg):
+    """The loop kernels' barrier: CTAs that wait for arrivals which never come leave after
+    the limit (one second here), CTAs that find the barrier given up leave at once."""
+    rc, waited_ms, later_ms = eik.selftest_grid_wait()
+    assert rc == 6, rc  # EIK_ERR_DEVICE: every wait expired and said so
+    assert 900.0 <= waited_ms <= 2000.0, waited_ms
+    assert later_ms <= 50.0, later_ms
+    e = _cube(eik, mg, 17, 3)[0]
+    e.solveEikonal()
+    first = e.getFinalResult().copy()
+    e.directLaunch_ = 1
+    e.solveEikonal()
+    assert bits_equal(first, e.getFinalResult())
+
+
 def _cube(eik, mg, n, seed):
     xyz, tets = mg.kuhn_cube(n, 0.2, seed=seed)
     v = mg.log_uniform_speeds(tets.shape[0], seed=seed + 1)
