@@ -3955,7 +3955,7 @@ size_t device_footprint(const Layout& L, const Built3D* b) {
   return nb * sizeof(BlockDesc) + ncoef * sizeof(float) + (size_t)L.total_slots * (sizeof(uint2) + sizeof(int)) +
          (L.dim == 3 ? (size_t)L.total_slots * (2 * sizeof(uint4) + sizeof(uint2)) : 0) + nhalo * sizeof(int) +
          ngraph * sizeof(int) +
-         nv * (2 * sizeof(int) + 5 * sizeof(float)) + nb * ((L.dim == 3 ? 12 : 9) * sizeof(int) + 1) + 7 * sizeof(int);
+         nv * (2 * sizeof(int) + 5 * sizeof(float)) + nb * (9 * sizeof(int) + 1) + 7 * sizeof(int);
 }
 
 cudaStream_t new_stream() {
