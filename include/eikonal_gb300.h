@@ -54,16 +54,24 @@ typedef struct eik_options {
   int verbose;             /* verbose_ (0) */
   int keep_history;        /* 1 (default): keep every iteration for eik_get_iteration */
   int fim_sweeps;          /* sweeps per active-block visit; -1 = reference (3D 2, 2D 7) */
-  int direct_launch;       /* 0 (default): a solve is one CUDA-graph launch; 1: the same kernels
-                              launched one by one with a host check per iteration, for profilers
-                              that cannot see kernels inside conditional graphs */
-  int threads_per_block;   /* CTA size of the 3D block-sweep kernels (128/256/384/512/768/1024).
-                              0 (default): 384 for the apex-item kernels (three CTAs per SM);
-                              for the slot kernels (precision mode, blocks too large for the
-                              item kernels' shared memory) chosen per handle over its first
-                              solves between one thread per slot of the largest block and 512,
-                              by measured speed.  Results do not depend on it.  The slot check
-                              kernel runs CTAs of half the size when this is 1024. */
+  int direct_launch;       /* 0 (default): with the reference's sweep counts a solve is one
+                              cooperative kernel for all of its iterations; in precision mode,
+                              with other sweep counts, with blocks too large for that kernel, and
+                              while other calls have work on the GPU that it would keep waiting,
+                              one CUDA graph.  1: the graph's kernels launched one by one with a
+                              host check per iteration, for profilers that cannot see kernels
+                              inside conditional graphs (they are not the cooperative kernel).
+                              Results do not depend on it. */
+  int threads_per_block;   /* CTA size of the 3D kernels (128/256/384/512/768/1024).  0 (default):
+                              in the cooperative kernel 768 threads up to 6 blocks per SM, 512 up
+                              to 24 and 384 beyond, in precision mode 768 and 384; 384 in the
+                              graph's other kernels.  For blocks too large for these kernels'
+                              shared memory, and in precision mode with other sweep counts, it is
+                              chosen per handle over its first solves between one thread per slot
+                              of the largest block and 512, by measured speed.  Results do not
+                              depend on it.  The slot check kernel runs CTAs of half the size when
+                              this is 1024.  It has no effect on the 2D kernels of up to 1024
+                              element slots a block. */
   int precision;           /* 0 (default): the reference's FP32 arithmetic, bit for bit.  1 (3D):
                               tets whose metric edge Gram matrix has condition number above
                               precision_kappa (slivers, strong anisotropy) run their local
@@ -82,7 +90,7 @@ typedef struct eik_options {
                               reference calls METIS 4 (so labels differ from the reference's);
                               EIK_ERR_ARG when the library was built without it.  Ignored when
                               is_structured is set or labels are given (eik_set_partition). */
-  int telemetry;           /* 1 (default): every launch of the loop records its span on the device
+  int telemetry;           /* 1 (default): every iteration of the loop records its span on the device
                               timer and its visit counts (eik_get_iteration_stats, the *_kernel_ms
                               and *_launches fields of eik_stats); 0: none of that, and the solve
                               runs about 1.5% faster on a 1.6M-tet mesh.  Results do not depend

@@ -3,7 +3,8 @@
 // One DeviceSolve owns the device copy of a block layout (slots, metric terms,
 // local vertex ids, halos, block graph) and the per-solve state (vertex travel
 // times, block flags, active lists, control block).  A solve is one launch of a
-// CUDA graph whose conditional while-node runs the reference's outer iteration
+// cooperative kernel, or of a CUDA graph whose conditional while-node runs the
+// reference's outer iteration
 // (src/core3d/cuda/meshFIM3dEikonal.cu:411-542, src/core2d/cuda/meshFIM2d_eikonal.cu:683-816)
 // entirely on the device: block visits, commit, neighbour activation and list
 // compaction, with no host round trip per iteration.

@@ -22,7 +22,7 @@
 // Design (GB300-first, not a translation):
 //   * A solve or batch of the reference's sweep counts is one cooperative launch whose
 //     CTAs stay for all iterations and meet at grid barriers.  Elsewhere (server,
-//     precision mode, other sweep counts) one CTA visits one block at a time: its own
+//     precision mode, other sweep counts, beside other calls) one CTA visits one block at a time: its own
 //     index first, then blocks from a device counter; grids are sized by occupancy x 152
 //     SMs and stay fixed so the whole iteration is a CUDA-graph body.  A conditional while-node repeats the
 //     body (four iterations a pass outside the server) until no block is active:
@@ -2515,9 +2515,11 @@ constexpr int kItemThreads = EIK_ITEM_THREADS;
 // gives none.  A mesh's blocks are active a fraction at a time: while fewer are than the
 // GPU holds CTAs, more warps per visit shorten it; when they fill the GPU, three visits
 // per SM overlap better.  Solves on one GB300 in us at 384 / 512 / 768 threads (three, two
-// and one CTA per SM): 562 blocks 1016 / 917 / 869, 792 blocks 1252 / 1117 / 1111, 1077
-// blocks 1423 / 1303 / 1359, 1839 blocks 1870 / 1812 / 2088, 2894 blocks 2325 / 2337 / 2885,
-// 4292 blocks 2776 / 2888 / 3763.
+// and one CTA per SM), 64 vertices and about 820 slots a block: 562 blocks 1016 / 917 / 869,
+// 792 blocks 1252 / 1117 / 1111, 1077 blocks 1423 / 1303 / 1359, 1839 blocks 1870 / 1812 /
+// 2088, 2894 blocks 2325 / 2337 / 2885, 4292 blocks 2776 / 2888 / 3763.  (Blocks of 4 to 32
+// vertices were not measured at each size; with this rule they take half the time that
+// 384 threads in the graph took.)
 int items_threads(int nb, int nsm, bool prec) {
   if (nb <= 6 * nsm) return 768;
   return (nb <= 24 * nsm && !prec) ? 512 : kItemThreads;

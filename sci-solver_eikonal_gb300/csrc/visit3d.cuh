@@ -292,8 +292,9 @@ __device__ __forceinline__ bool check_visit3d(const DevArgs& a, const BlockDesc&
 }
 
 // The two sweeps of a loaded block (its sweep memos in h0, or behind a check read from
-// memory, where `memo` says they are of this solve): the final owned times in v2, those after the first sweep in v1.  s_n as above.
-// Ends behind a CTA barrier.
+// memory, where `memo` says they are of this solve): the final owned times in v2, those
+// after the first sweep in v1, both behind a CTA barrier.  s_n: counters that are zero
+// again only behind the caller's next barrier.
 template <bool kPrec = false>
 __device__ __forceinline__ void sweep_visit3d(const DevArgs& a, const BlockDesc& bd, const SmemV& s, int* s_n,
                                               bool checked, bool memo, PrecMode pm = PrecMode{0, 0}) {
